@@ -263,12 +263,11 @@ __device__ __forceinline__ FFTTabs fft_tabs_init(unsigned char* base, const FFTP
 template <int G>
 __device__ __forceinline__ int ppos(int k) { return k + k / G; }
 
-// Column pass over `nrows` rows of stride RS = E (G + 1).  SIGN +1 (inverse): E-point DFT
+// Column pass over `nrows` rows of stride RS (E (G + 1), or more).  SIGN +1 (inverse): E-point DFT
 // over k2 of Z[k1 + G k2], then the twiddle w^(t1 k1).  SIGN -1 (forward): the twiddle
 // w^(-t1 k1) first, then the E-point DFT.  In place.
-template <int E, int G, int SIGN>
+template <int E, int G, int SIGN, int RS = E * (G + 1)>
 __device__ __forceinline__ void col_pass(double2* rows, int nrows, const FFTTabs& t) {
-  constexpr int RS = E * (G + 1);
   for (int i = threadIdx.x; i < nrows * G; i += blockDim.x) {
     const int r = i / G, k1 = i - r * G;
     double2* col = rows + (size_t)r * RS + k1;
@@ -290,9 +289,8 @@ __device__ __forceinline__ void col_pass(double2* rows, int nrows, const FFTTabs
 }
 
 // Row pass: a G-point DFT over the G contiguous values of each (row, t1).  In place.
-template <int E, int G, int SIGN>
+template <int E, int G, int SIGN, int RS = E * (G + 1)>
 __device__ __forceinline__ void row_pass(double2* rows, int nrows, const FFTTabs& t) {
-  constexpr int RS = E * (G + 1);
   for (int i = threadIdx.x; i < nrows * E; i += blockDim.x) {
     const int r = i / E, t1 = i - r * E;
     double2* seg = rows + (size_t)r * RS + t1 * (G + 1);
@@ -332,21 +330,6 @@ __device__ __forceinline__ void st_global_2c(cplx* p, double2 a, double2 b) {
 
 // theta row of half-row h on side 0 (south) / 1 (north)
 __device__ __forceinline__ int row_theta(int h, int side, int Th) { return side ? Th - 1 - h : h; }
-
-// A staged field: the folded rows of the CTA's half-row pair in bin order,
-// sp[(p * 2 + jj) * M + b] (p = E/O).  Row (jj, side): Y = E + O (south), E - O (north);
-// bins b >= M are zero.
-__device__ __forceinline__ double2 row_bin(const double2* sp, int b, int jj, int side, int M) {
-  if (b >= M) return make_double2(0.0, 0.0);
-  const double2 e = sp[jj * M + b], o = sp[(2 + jj) * M + b];
-  return side ? sub2(e, o) : add2(e, o);
-}
-
-// stage element i (raw order (c, p, jj)) of one field's (n, h/2) block into bin order
-__device__ __forceinline__ void stage_elem(double2* sp, const cplx* blk, const FFTTabs& t, int M, int i) {
-  const int c = i >> 2, p = (i >> 1) & 1, jj = i & 1;
-  sp[(p * 2 + jj) * M + t.thm[c]] = blk[i];
-}
 
 // bin b < M of a transformed row (natural order, padded) as a real-spectrum bin
 template <int G>
@@ -689,77 +672,116 @@ __global__ void __launch_bounds__(PROD_THREADS, 2) k_products(FFTPlanDev pl, int
   }
 }
 
-// ---- standalone c2r: theta-Fourier -> phys [f][n][Ph][Th] -------------------------------
-// grid (HB, N, nfields), 128 threads: the four theta rows of a half-row pair.
+// ---- standalone transforms between theta-Fourier rows and phys [f][n][Ph][Th] -------------
+// The grid is contiguous along theta, the transforms run along phi.  A CTA takes HT half-rows,
+// so its southern and its northern rows are HT neighbours each in theta: HT = 8 (64-byte
+// segments) while 16 rows fit three CTAs' shared memory, else 4 (32-byte sectors), and the lanes
+// of a warp run along theta first.  What bounds them is HBM: at lmax 255 (8 x 64 shells, 0.81 GB
+// of theta-Fourier rows, 1.21 GB of grid) c2r takes 0.79 ms and r2c 0.98 ms; with two half-rows a
+// CTA and a lane per phi sample (8-byte accesses a theta row apart) they took 2.08 and 1.58 ms.
+// Rows lie side-major ([side][HT]); their stride RSP is E (G + 1) padded so that the 8 lanes
+// of a 128-byte shared-memory access (HT rows x 8 / HT samples, which are G + 1 apart) fall in
+// distinct banks: RSP = 1 mod 2 (HT = 8), 2 mod 8 (HT = 4).
+template <int E, int G> struct GridTile {
+  static constexpr int RS = E * (G + 1);
+  static constexpr int HT = 16 * (RS + 1) * (int)sizeof(double2) <= 56 * 1024 ? 8 : 4;
+  static constexpr int RSP = HT == 8 ? RS | 1 : RS + (10 - RS % 8) % 8;
+  static constexpr int THREADS = 32 * HT;  // one column DFT a thread at G = 16
+  static constexpr int MINB = E > 24 ? 1 : HT == 8 && E > 12 ? 2 : 3;
+};
+
+// 64 bytes (E, O of both half-rows of a pair: four_off) as two 32-byte loads
+__device__ __forceinline__ void ld_pair(const cplx* p, double2 (&v)[4]) {
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(v[0].x), "=d"(v[0].y), "=d"(v[1].x), "=d"(v[1].y) : "l"(p));
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(v[2].x), "=d"(v[2].y), "=d"(v[3].x), "=d"(v[3].y) : "l"(p + 2));
+}
+
+// c2r; grid (ceil(Th2 / HT), N, nfields)
 template <int E, int G>
-__global__ void __launch_bounds__(128) k_c2r(FFTPlanDev pl, int N, const cplx* four, double* phys) {
-  constexpr int RS = E * (G + 1), P2 = E * G;
+__global__ void __launch_bounds__(GridTile<E, G>::THREADS, GridTile<E, G>::MINB)
+    k_c2r(FFTPlanDev pl, int N, const cplx* four, double* phys) {
+  constexpr int HT = GridTile<E, G>::HT, RSP = GridTile<E, G>::RSP, P2 = E * G, KH = P2 / 2 + 1;
+  constexpr int NTHR = GridTile<E, G>::THREADS;
   extern __shared__ __align__(16) unsigned char csm[];
-  const int hb = blockIdx.x, n = blockIdx.y, f = blockIdx.z;
-  const int Th = pl.Th, Th2 = pl.Th2, M = pl.M, NM = pl.NM;
-  double2* rows = (double2*)csm;    // [4][RS]
-  double2* sp = rows + 4 * RS;      // [4][M]
-  const FFTTabs tabs = fft_tabs_init<E, G>((unsigned char*)(sp + 4 * M), pl);
-  const cplx* blk = four + (((size_t)f * N + n) * pl.HB + hb) * NM * 4;
-  for (int i = threadIdx.x; i < NM * 4; i += blockDim.x) stage_elem(sp, blk, tabs, M, i);
-  __syncthreads();
-  for (int i = threadIdx.x; i < 4 * P2; i += blockDim.x) {
-    const int r = i / P2, k = i - r * P2;
-    rows[r * RS + ppos<G>(k)] = c2r_pack(k, row_bin(sp, k, r >> 1, r & 1, M), row_bin(sp, k == 0 ? P2 : P2 - k, r >> 1, r & 1, M), tabs.twh);
+  const int h0 = blockIdx.x * HT, n = blockIdx.y, f = blockIdx.z;
+  const int Th = pl.Th, Th2 = pl.Th2, M = pl.M, NM = pl.NM, HB = pl.HB;
+  double2* rows = (double2*)csm;  // [2 sides][HT][RSP]
+  const FFTTabs tabs = fft_tabs_init<E, G>((unsigned char*)(rows + 2 * HT * RSP), pl);
+  const cplx* blk = four + ((size_t)f * N + n) * HB * NM * 4;
+  // item (half-row pair q, k): bins k and P2 - k of the pair's two half-rows, packed into their
+  // four rows at k and P2 - k (bins >= M are zero)
+  for (int i = threadIdx.x; i < HT / 2 * KH; i += NTHR) {
+    const int q = i / KH, k = i - q * KH, km = k == 0 ? P2 : P2 - k, hb = h0 / 2 + q;
+    if (hb >= HB) break;  // past the last pair (q grows with i)
+    double2 a[4], b[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) a[j] = b[j] = make_double2(0.0, 0.0);
+    if (k < M) ld_pair(blk + ((size_t)hb * NM + tabs.b2c[k]) * 4, a);
+    if (km < M) ld_pair(blk + ((size_t)hb * NM + tabs.b2c[km]) * 4, b);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {  // r = side 2 + h % 2
+      const int jj = r & 1;
+      const double2 yk = r < 2 ? add2(a[jj], a[2 + jj]) : sub2(a[jj], a[2 + jj]);
+      const double2 ym = r < 2 ? add2(b[jj], b[2 + jj]) : sub2(b[jj], b[2 + jj]);
+      double2* row = rows + ((r >> 1) * HT + 2 * q + jj) * RSP;
+      row[ppos<G>(k)] = c2r_pack(k, yk, ym, tabs.twh);
+      if (k != 0 && 2 * k != P2) row[ppos<G>(P2 - k)] = c2r_pack(P2 - k, ym, yk, tabs.twh);
+    }
   }
   __syncthreads();
-  col_pass<E, G, +1>(rows, 4, tabs);
+  col_pass<E, G, +1, RSP>(rows, 2 * HT, tabs);
   __syncthreads();
-  row_pass<E, G, +1>(rows, 4, tabs);
+  row_pass<E, G, +1, RSP>(rows, 2 * HT, tabs);
   __syncthreads();
   double* dst = phys + ((size_t)f * N + n) * (size_t)pl.Ph * Th;
-  for (int i = threadIdx.x; i < 4 * P2; i += blockDim.x) {
-    const int r = i / P2, pos = i - r * P2;       // pos = (G+1) t1 + t2 without the pads
-    const int t1 = pos / G, t2 = pos - t1 * G, t = t1 + E * t2;
-    const int h = 2 * hb + (r >> 1), side = r & 1;
-    if (h >= Th2) continue;
-    const int j = row_theta(h, side, Th);
-    if (side && j == h) continue;  // odd Th: the equator row is written once
-    const double2 z = rows[r * RS + t1 * (G + 1) + t2];
-    dst[(size_t)(2 * t) * Th + j] = z.x;
-    dst[(size_t)(2 * t + 1) * Th + j] = z.y;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < 2 * HT * P2; i += NTHR) {
+    const int jl = i % HT, ts = i / HT, side = ts / P2, t = ts - side * P2, t2 = t / E, t1 = t - t2 * E;
+    const int h = h0 + jl, j = row_theta(h, side, Th);
+    if (h < Th2 && !(side && j == h)) {  // odd Th: the equator row is written once
+      const double2 z = rows[(side * HT + jl) * RSP + t1 * (G + 1) + t2];
+      dst[(size_t)(2 * t) * Th + j] = z.x;
+      dst[(size_t)(2 * t + 1) * Th + j] = z.y;
+    }
   }
 }
 
-// ---- standalone r2c: phys [f][n][Ph][Th] -> folded theta-Fourier, analysis layout ---------
+// r2c: phys -> folded theta-Fourier rows, analysis layout; grid (ceil(Th2 / HT), N, nfields)
 template <int E, int G>
-__global__ void __launch_bounds__(128) k_r2c(FFTPlanDev pl, int N, const double* phys, cplx* four) {
-  constexpr int RS = E * (G + 1), P2 = E * G;
+__global__ void __launch_bounds__(GridTile<E, G>::THREADS, GridTile<E, G>::MINB)
+    k_r2c(FFTPlanDev pl, int N, const double* phys, cplx* four) {
+  constexpr int HT = GridTile<E, G>::HT, RSP = GridTile<E, G>::RSP, P2 = E * G;
+  constexpr int NTHR = GridTile<E, G>::THREADS;
   extern __shared__ __align__(16) unsigned char rsm[];
-  const int hb = blockIdx.x, n = blockIdx.y, f = blockIdx.z;
+  const int h0 = blockIdx.x * HT, n = blockIdx.y, f = blockIdx.z;
   const int Th = pl.Th, Th2 = pl.Th2, NM = pl.NM;
-  double2* rows = (double2*)rsm;  // [4][RS]
-  const FFTTabs tabs = fft_tabs_init<E, G>((unsigned char*)(rows + 4 * RS), pl);
+  double2* rows = (double2*)rsm;  // [2 sides][HT][RSP]
+  const FFTTabs tabs = fft_tabs_init<E, G>((unsigned char*)(rows + 2 * HT * RSP), pl);
   const double scale = 1.0 / (double)pl.Ph;
   const double* src = phys + ((size_t)f * N + n) * (size_t)pl.Ph * Th;
-  for (int i = threadIdx.x; i < 4 * P2; i += blockDim.x) {
-    const int r = i / P2, pos = i - r * P2;
-    const int t1 = pos / G, t2 = pos - t1 * G, t = t1 + E * t2;
-    const int h = 2 * hb + (r >> 1);
-    const int j = row_theta(h < Th2 ? h : 2 * hb, r & 1, Th);
-    rows[r * RS + t1 * (G + 1) + t2] =
-        make_double2(src[(size_t)(2 * t) * Th + j] * scale, src[(size_t)(2 * t + 1) * Th + j] * scale);
+#pragma unroll 8
+  for (int i = threadIdx.x; i < 2 * HT * P2; i += NTHR) {
+    const int jl = i % HT, ts = i / HT, side = ts / P2, t = ts - side * P2, t2 = t / E, t1 = t - t2 * E;
+    const int h = h0 + jl, j = row_theta(h < Th2 ? h : Th2 - 1, side, Th);
+    const double* p = src + (size_t)(2 * t) * Th + j;
+    rows[(side * HT + jl) * RSP + t1 * (G + 1) + t2] = make_double2(__ldg(p) * scale, __ldg(p + Th) * scale);
   }
   __syncthreads();
-  row_pass<E, G, -1>(rows, 4, tabs);
+  row_pass<E, G, -1, RSP>(rows, 2 * HT, tabs);
   __syncthreads();
-  col_pass<E, G, -1>(rows, 4, tabs);
+  col_pass<E, G, -1, RSP>(rows, 2 * HT, tabs);
   __syncthreads();
   cplx* fld = four + (size_t)f * N * pl.HB * NM * 4;  // analysis layout (four_off_a)
-  for (int i = threadIdx.x; i < NM * 2; i += blockDim.x) {
-    const int c = i >> 1, q = i & 1, hh = 2 * hb + q, b = tabs.thm[c];
-    if (hh >= Th2) continue;
-    const double2 xs = row_unpack<G>(rows + (2 * q) * RS, b, P2, tabs.twh);
-    const double2 xn = row_unpack<G>(rows + (2 * q + 1) * RS, b, P2, tabs.twh);
+  for (int i = threadIdx.x; i < NM * HT; i += NTHR) {  // a counter's HT (E, O) pairs are contiguous
+    const int hl = i % HT, c = i / HT, h = h0 + hl, b = tabs.thm[c];
+    if (h >= Th2) continue;
+    const double2 xs = row_unpack<G>(rows + hl * RSP, b, P2, tabs.twh);
+    const double2 xn = row_unpack<G>(rows + (HT + hl) * RSP, b, P2, tabs.twh);
     double2 ev = add2(xs, xn);
-    if ((Th & 1) && hh == Th2 - 1) { ev.x *= 0.5; ev.y *= 0.5; }
-    fld[four_off_a(n, c, 0, hh, N, Th2)] = ev;
-    fld[four_off_a(n, c, 1, hh, N, Th2)] = sub2(xs, xn);
+    if ((Th & 1) && h == Th2 - 1) { ev.x *= 0.5; ev.y *= 0.5; }
+    st_global_2c(fld + four_off_a(n, c, 0, h, N, Th2), ev, sub2(xs, xn));
   }
 }
 
@@ -836,40 +858,41 @@ bool lsd_fft_plan(lsd_ctx* c) {
   return dispatch_EG(E, G, [](auto, auto) { return 0; }) == 0;
 }
 
-int lsd_launch_c2r(lsd_ctx* ctx, const cplx* four, double* phys, int nfields) {
-  FFTPlanDev pl = make_plan(ctx);
-  dim3 grid(ctx->HB, ctx->N, nfields);
-  const size_t smem = sizeof(double2) * 4 * (ctx->fftE * (ctx->fftG + 1) + ctx->M) +
-                      fft_tab_bytes(ctx->P2, ctx->fftE, ctx->fftG, ctx->NM);
+namespace {
+// one launch of a grid transform: f(kernel<E, G>)'s grid, threads and shared memory
+template <class KERN>
+int launch_grid_fft(lsd_ctx* ctx, const char* name, int nfields, KERN&& launch) {
   int rc = dispatch_EG(ctx->fftE, ctx->fftG, [&](auto e, auto g) {
     constexpr int E = decltype(e)::value, G = decltype(g)::value;
-    cudaFuncSetAttribute(k_c2r<E, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_c2r<E, G><<<grid, 128, smem, ctx->stream>>>(pl, ctx->N, four, phys);
+    using T = GridTile<E, G>;
+    const size_t smem = sizeof(double2) * 2 * T::HT * T::RSP + fft_tab_bytes(ctx->P2, E, G, ctx->NM);
+    launch(e, g, dim3(ceil_div(ctx->Th2, T::HT), ctx->N, nfields), T::THREADS, smem);
     return 0;
   });
   if (rc) return lsd_fail(ctx, LSD_EARG, "FFT length not supported");
   ctx->launches++;
   cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return lsd_fail(ctx, LSD_ECUDA, std::string("k_c2r: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) return lsd_fail(ctx, LSD_ECUDA, std::string(name) + ": " + cudaGetErrorString(e));
   return LSD_OK;
+}
+}  // namespace
+
+int lsd_launch_c2r(lsd_ctx* ctx, const cplx* four, double* phys, int nfields) {
+  const FFTPlanDev pl = make_plan(ctx);
+  return launch_grid_fft(ctx, "k_c2r", nfields, [&](auto e, auto g, dim3 grid, int threads, size_t smem) {
+    constexpr int E = decltype(e)::value, G = decltype(g)::value;
+    cudaFuncSetAttribute(k_c2r<E, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_c2r<E, G><<<grid, threads, smem, ctx->stream>>>(pl, ctx->N, four, phys);
+  });
 }
 
 int lsd_launch_r2c(lsd_ctx* ctx, const double* phys, cplx* four, int nfields) {
-  FFTPlanDev pl = make_plan(ctx);
-  dim3 grid(ctx->HB, ctx->N, nfields);
-  const size_t smem = sizeof(double2) * 4 * ctx->fftE * (ctx->fftG + 1) +
-                      fft_tab_bytes(ctx->P2, ctx->fftE, ctx->fftG, ctx->NM);
-  int rc = dispatch_EG(ctx->fftE, ctx->fftG, [&](auto e, auto g) {
+  const FFTPlanDev pl = make_plan(ctx);
+  return launch_grid_fft(ctx, "k_r2c", nfields, [&](auto e, auto g, dim3 grid, int threads, size_t smem) {
     constexpr int E = decltype(e)::value, G = decltype(g)::value;
     cudaFuncSetAttribute(k_r2c<E, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_r2c<E, G><<<grid, 128, smem, ctx->stream>>>(pl, ctx->N, phys, four);
-    return 0;
+    k_r2c<E, G><<<grid, threads, smem, ctx->stream>>>(pl, ctx->N, phys, four);
   });
-  if (rc) return lsd_fail(ctx, LSD_EARG, "FFT length not supported");
-  ctx->launches++;
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return lsd_fail(ctx, LSD_ECUDA, std::string("k_r2c: ") + cudaGetErrorString(e));
-  return LSD_OK;
 }
 
 namespace {
