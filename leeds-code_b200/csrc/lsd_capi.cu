@@ -38,7 +38,7 @@ void free_ctx(lsd_ctx* ctx) {
     cudaEventDestroy(x.fork);
   }
   lsd_ozaki_free(ctx);
-  void* ptrs[] = {ctx->d_sblk_l, ctx->d_sblk_nh, ctx->d_aperm, ctx->d_l, ctx->d_m, ctx->d_s, ctx->d_mc, ctx->d_mstart, ctx->d_mlen, ctx->d_thm, ctx->d_bin2c, ctx->d_lm2nh,
+  void* ptrs[] = {ctx->d_l, ctx->d_m, ctx->d_s, ctx->d_mc, ctx->d_mstart, ctx->d_mlen, ctx->d_thm, ctx->d_bin2c, ctx->d_lm2nh,
                   ctx->d_leg, ctx->d_gp, ctx->d_gw, ctx->d_sn, ctx->d_sn1, ctx->d_tw2, ctx->d_twh, ctx->d_r,
                   ctx->d_dr, ctx->d_r1dr, ctx->d_radlap, ctx->d_intr2dr, ctx->d_lu, ctx->d_lus, ctx->d_y, ctx->d_yt,
                   ctx->d_ipiv, ctx->d_ipivs, ctx->d_info, ctx->d_gre, ctx->d_gret, ctx->d_invg, ctx->d_state, ctx->d_nl,
@@ -595,32 +595,6 @@ int lsd_create(const lsd_config* cfg, lsd_ctx** out) {
     TRY(dalloc(ctx, &ctx->d_bin2c, b2c.size())); TRY(upload(ctx, ctx->d_bin2c, b2c));
   }
   TRY(dalloc(ctx, &ctx->d_lm2nh, lm2nh.size())); TRY(upload(ctx, ctx->d_lm2nh, lm2nh));
-  {  // analysis thread order per folded column: (m-counter, parity)-sorted harmonics
-    std::vector<int> perm((size_t)ctx->Hc * ctx->Hr);
-    for (int col = 0; col < ctx->Hc; ++col) {
-      int base = col * ctx->Hr, len0 = ctx->mlen[2 * col], t = 0;
-      for (int cl = 0; cl < 2; ++cl)
-        for (int par = 0; par < 2; ++par)
-          for (int k = 0; k < ctx->Hr; ++k)
-            if ((k < len0 ? 0 : 1) == cl && ctx->hs[base + k] == par) perm[(size_t)col * ctx->Hr + t++] = k;
-    }
-    TRY(dalloc(ctx, &ctx->d_aperm, perm.size())); TRY(upload(ctx, ctx->d_aperm, perm));
-  }
-  {  // solve blocks: one degree l, up to 16 orders m (all (l, m) share the factors of l)
-    std::vector<int> bl, bnh;
-    for (int l = 0; l < L; ++l) {
-      std::vector<int> nhs;
-      for (int mi = 0; mi < ctx->M; ++mi)
-        if (lm2nh[(size_t)mi * L + l] >= 0) nhs.push_back(lm2nh[(size_t)mi * L + l]);
-      for (size_t i0 = 0; i0 < nhs.size(); i0 += 16) {
-        bl.push_back(l);
-        for (size_t i = i0; i < i0 + 16; ++i) bnh.push_back(i < nhs.size() ? nhs[i] : -1);
-      }
-    }
-    ctx->nsblk = (int)bl.size();
-    TRY(dalloc(ctx, &ctx->d_sblk_l, bl.size())); TRY(upload(ctx, ctx->d_sblk_l, bl));
-    TRY(dalloc(ctx, &ctx->d_sblk_nh, bnh.size())); TRY(upload(ctx, ctx->d_sblk_nh, bnh));
-  }
   // FFT twiddles (long double host trigonometry, rounded once)
   {
     std::vector<double2> tw2(ctx->P2), twh(ctx->Ph);

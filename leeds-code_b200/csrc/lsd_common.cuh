@@ -112,9 +112,6 @@ struct lsd_ctx {
   // device layout
   int *d_l = nullptr, *d_m = nullptr, *d_s = nullptr, *d_mc = nullptr;
   int *d_mstart = nullptr, *d_mlen = nullptr, *d_thm = nullptr, *d_lm2nh = nullptr, *d_bin2c = nullptr;
-  int *d_aperm = nullptr;  // [Hc][Hr] analysis thread order
-  int *d_sblk_l = nullptr, *d_sblk_nh = nullptr;  // solve blocks: degree, [16] harmonics
-  int nsblk = 0;
   int nh_l1m0 = -1, nh_l1m1 = -1;  // toroidal modes of vel_angmomclr
   // device Legendre tables, each [H][Th2] (== Fortran (Th2, H))
   double *d_leg = nullptr;  // 8 tables contiguous, LSD_LEG_* order

@@ -8,332 +8,254 @@
 // (transform.fftw3.F90:527-602, 825-949).
 //
 // Data layouts: spectral [n][H] complex (harmonic fastest, the reference's `spec`
-// order); theta-Fourier rows folded into even/odd half-grid sums: synthesis writes them in
-// half-row pairs for the FFT (four_off: [n][h/2][m-counter][E/O][h%2]), analysis reads them
-// counter-major (four_off_a: [m-counter][n][h][E/O]);
-// tables [nh][Th2] (the reference's leg_*(Th2, 0:H-1)).
+// order; the harmonics of an m-counter are contiguous, l ascending from m, so parity
+// (l + m) mod 2 alternates along them); theta-Fourier rows folded into even/odd half-grid
+// sums: synthesis writes them in half-row pairs for the FFT (four_off:
+// [n][h/2][m-counter][E/O][h%2]), analysis reads them counter-major (four_off_a:
+// [m-counter][n][h][E/O]); tables [nh][Th2] (the reference's leg_*(Th2, 0:H-1)).
 //
-// Synthesis CTA = (m-counter, NT shells, group); thread = one theta row j of the half
-// grid, holding E/O accumulators for NT shells x 3 outputs; coefficients of the current
-// k-chunk are smem broadcasts, table rows are read conflict-free along j.
-// Analysis CTA = (folded column = two m-counters, NT shells, group); thread = one
-// harmonic k of the column; the folded (E/O) data of a j-chunk are smem broadcasts.
+// Both directions are real matrix products per (m-counter, parity): M = theta rows
+// (synthesis) or harmonics (analysis), K = harmonics or theta rows, columns = (shell, Re / Im
+// of the outputs).  They run on the FP64 tensor instruction m8n8k4, whose products and sums
+// are IEEE FP64 fused multiply-adds at the card's full FP64 rate (36.8 TF/s here, FFMA code
+// 34.1) with a third of the operand reads of a thread-tiled product.
+//
+// A CTA (4 warps) takes one counter, 48 M rows and 64 columns; warp = (parity, column half),
+// a tile of 6 x 4 m8n8 accumulators.  Both parities of a counter share the staged data, since
+// every value enters one parity directly and (vector transforms) the other one crosswise:
+//   vector  out0 = a0 T1 (other parity) - i a1 T2 (own), out1 = a1 T1 + i a0 T2
+//   scalar  out = a T (own parity; the output's label flips for the theta derivative)
+// K runs in chunks of 8 + 8 (both parities) through a three-stage ring of asynchronous
+// copies (16-byte, 8-byte where an odd Th2 misaligns the tables), three CTAs per SM.  What bounds
+// it: the FP64 tensor pipe at large L, the ring's first fill where a counter has few K.
+// At lmax 127, Nr 129 (one evaluation: 4 vector syntheses and a gradient, 2 vector and a scalar
+// analysis) 0.53 ms at 57 % of the pipe and 0.32 ms at 76 %; thread-tiled products with a theta row
+// or a harmonic per thread took 3.37 and 1.40 ms (2.8 and 3.2 TF/s, waiting for their tables).
 #include "lsd_common.cuh"
 
 namespace {
 
-constexpr int S_NT = 4;   // shells per synthesis CTA
-constexpr int S_KC = 16;  // harmonics per synthesis k-chunk
-constexpr int A_NT = 8;   // shells per analysis CTA
-constexpr int A_JC = 16;  // theta rows per analysis j-chunk
-constexpr int DROW = A_JC * A_NT + 1;  // padded analysis data row (double2)
+constexpr int LG_MT = 6, LG_BM = 8 * LG_MT;  // m8 tiles and M rows of a CTA
+constexpr int LG_NT = 4;                     // n8 tiles of a warp (32 columns)
+constexpr int LG_STAGES = 3, LG_THREADS = 128;
+constexpr int LG_MAXG = 8, LG_MAXCLASS = 4;
+// shared-memory strides, chosen so that the 16 lanes of a 128-byte access of a fragment read
+// (4 along K x 4 along the other index) fall in distinct banks:
+constexpr int LG_DROW = 17;   // complex per staged (shell, field) row: 16 = 8 K x 2 parities
+constexpr int LG_AS = 50;     // synthesis: doubles per table row [kk][48 theta]
+constexpr int LG_AA = 10;     // analysis: doubles per table row [harmonic][8 theta]
+constexpr int LG_DATA = 32 * LG_DROW * 2;           // doubles of a stage's data
+constexpr int LG_TAB_S = 16 * LG_AS, LG_TAB_A = 2 * LG_BM * LG_AA;  // ... of one table tile
 
-struct SynthArgs {
-  int N, H, Th, Th2, NM, HB, ngroup;
+// Groups of one launch that share tables: vec: two fields per group, tables T1 (other parity)
+// and T2 (own); scalar: one field, table tab[0].
+struct LegClass {
+  int vec, tab[2];
+  int flip, rot, scale;  // scalar synthesis: output parity flipped; times i; times 1/r
+  int ng;
+  unsigned zero;         // analysis: bit g: drop the imaginary part of m = 0
+  const cplx* in[2][LG_MAXG];
+  cplx* out[2][LG_MAXG];
+};
+struct LegArgs {
+  int N, H, Th2, NM, HB, mtiles;
   const int* mstart;
   const int* mlen;
-  const int* hs;
-  const double* leg;  // 8 tables [t][H][Th2]
-  const double* rinv; // 1/r per shell
-  SynthGroup g[6];
-};
-
-__device__ __forceinline__ double2 cmul_i(double2 a) { return make_double2(-a.y, a.x); }     // i*a
-__device__ __forceinline__ double2 cmul_mi(double2 a) { return make_double2(a.y, -a.x); }    // -i*a
-
-// KIND-specific: number of inputs, outputs and tables used
-template <int KIND> struct SK;
-template <> struct SK<SK_VECTOR> { static constexpr int nin = 3, nout = 3, ntab = 3; };
-template <> struct SK<SK_SCALAR> { static constexpr int nin = 1, nout = 1, ntab = 1; };
-template <> struct SK<SK_GRAD3> { static constexpr int nin = 2, nout = 3, ntab = 3; };
-template <> struct SK<SK_GRAD2> { static constexpr int nin = 1, nout = 2, ntab = 2; };
-
-template <int KIND>
-__device__ __forceinline__ int synth_table(int t) {
-  if (KIND == SK_VECTOR) return t == 0 ? LSD_LEG_P : (t == 1 ? LSD_LEG_LLP_ : LSD_LEG_LLSIN1MP);
-  if (KIND == SK_SCALAR) return LSD_LEG_P;
-  if (KIND == SK_GRAD3) return t == 0 ? LSD_LEG_P : (t == 1 ? LSD_LEG_P_ : LSD_LEG_SIN1MP);
-  return t == 0 ? LSD_LEG_P_ : LSD_LEG_SIN1MP;  // SK_GRAD2
-}
-
-// One harmonic k of the current chunk: accumulate into the even (E) / odd (O) sums of
-// the outputs; S = parity of (l + m) of this harmonic.
-template <int KIND, int S, int NOUT>
-__device__ __forceinline__ void synth_accum(double2 (&acc)[NOUT][2][S_NT], const double* tab,
-                                            const double2* coef, int kk, int j, int Th2) {
-  constexpr int O = 1 - S;
-  if (KIND == SK_VECTOR) {
-    const double P = tab[(0 * S_KC + kk) * Th2 + j];
-    const double A1 = tab[(1 * S_KC + kk) * Th2 + j];
-    const double A2 = tab[(2 * S_KC + kk) * Th2 + j];
-#pragma unroll
-    for (int q = 0; q < S_NT; ++q) {
-      const double2 cq = coef[(0 * S_KC + kk) * S_NT + q];
-      const double2 cs = coef[(1 * S_KC + kk) * S_NT + q];
-      const double2 ct = coef[(2 * S_KC + kk) * S_NT + q];
-      const double2 c2 = cmul_mi(ct);  // (t.Im, -t.Re)
-      const double2 c3 = cmul_i(cs);   // (-s.Im, s.Re)
-      // r: P on parity S ; th: llP_ on 1-S, llsin1mP on S ; ph: llsin1mP on S, llP_ on 1-S
-      acc[0][S][q].x += cq.x * P;  acc[0][S][q].y += cq.y * P;
-      acc[1][O][q].x += cs.x * A1; acc[1][O][q].y += cs.y * A1;
-      acc[1][S][q].x += c2.x * A2; acc[1][S][q].y += c2.y * A2;
-      acc[2][S][q].x += c3.x * A2; acc[2][S][q].y += c3.y * A2;
-      acc[2][O][q].x += ct.x * A1; acc[2][O][q].y += ct.y * A1;
-    }
-  } else if (KIND == SK_SCALAR) {
-    const double P = tab[kk * Th2 + j];
-#pragma unroll
-    for (int q = 0; q < S_NT; ++q) {
-      const double2 cq = coef[kk * S_NT + q];
-      acc[0][S][q].x += cq.x * P; acc[0][S][q].y += cq.y * P;
-    }
-  } else if (KIND == SK_GRAD3) {
-    const double P = tab[(0 * S_KC + kk) * Th2 + j];
-    const double D = tab[(1 * S_KC + kk) * Th2 + j];
-    const double S1 = tab[(2 * S_KC + kk) * Th2 + j];
-#pragma unroll
-    for (int q = 0; q < S_NT; ++q) {
-      const double2 cd = coef[(0 * S_KC + kk) * S_NT + q];
-      const double2 cc = coef[(1 * S_KC + kk) * S_NT + q];
-      const double2 ci = cmul_i(cc);
-      acc[0][S][q].x += cd.x * P;  acc[0][S][q].y += cd.y * P;
-      acc[1][O][q].x += cc.x * D;  acc[1][O][q].y += cc.y * D;
-      acc[2 % NOUT][S][q].x += ci.x * S1; acc[2 % NOUT][S][q].y += ci.y * S1;
-    }
-  } else {  // SK_GRAD2
-    const double D = tab[(0 * S_KC + kk) * Th2 + j];
-    const double S1 = tab[(1 * S_KC + kk) * Th2 + j];
-#pragma unroll
-    for (int q = 0; q < S_NT; ++q) {
-      const double2 cc = coef[kk * S_NT + q];
-      const double2 ci = cmul_i(cc);
-      acc[0][O][q].x += cc.x * D;  acc[0][O][q].y += cc.y * D;
-      acc[1 % NOUT][S][q].x += ci.x * S1; acc[1 % NOUT][S][q].y += ci.y * S1;
-    }
-  }
-}
-
-template <int KIND>
-__global__ void __launch_bounds__(256) k_synth(SynthArgs a) {
-  constexpr int NIN = SK<KIND>::nin, NOUT = SK<KIND>::nout, NTAB = SK<KIND>::ntab;
-  extern __shared__ double smem[];
-  const int c = blockIdx.x;
-  const int n0 = blockIdx.y * S_NT;
-  const SynthGroup& G = a.g[blockIdx.z];
-  const int Th2 = a.Th2;
-  const int kbeg = a.mstart[c], klen = a.mlen[c];
-  double* tab = smem;                                   // [NTAB][S_KC][Th2]
-  double2* coef = (double2*)(smem + NTAB * S_KC * Th2); // [NIN][S_KC][S_NT]
-  __shared__ int spar[S_KC];
-  const int j = threadIdx.x;
-  // accumulators acc[out][parity][shell]
-  double2 acc[NOUT][2][S_NT];
-#pragma unroll
-  for (int o = 0; o < NOUT; ++o)
-#pragma unroll
-    for (int p = 0; p < 2; ++p)
-#pragma unroll
-      for (int q = 0; q < S_NT; ++q) acc[o][p][q] = make_double2(0.0, 0.0);
-
-  for (int k0 = 0; k0 < klen; k0 += S_KC) {
-    const int kc = min(S_KC, klen - k0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < NTAB * kc * Th2; i += blockDim.x) {
-      int t = i / (kc * Th2), rem = i % (kc * Th2), kk = rem / Th2, jj = rem % Th2;
-      tab[(t * S_KC + kk) * Th2 + jj] =
-          a.leg[(size_t)synth_table<KIND>(t) * a.H * Th2 + (size_t)(kbeg + k0 + kk) * Th2 + jj];
-    }
-    for (int i = threadIdx.x; i < NIN * kc * S_NT; i += blockDim.x) {
-      int f = i / (kc * S_NT), rem = i % (kc * S_NT), q = rem / kc, kk = rem % kc;
-      int n = n0 + q;
-      double2 v = make_double2(0.0, 0.0);
-      if (n < a.N) {
-        v = G.in[f][(size_t)n * a.H + kbeg + k0 + kk];
-        if (KIND == SK_GRAD3 && f == 1) { double r1 = a.rinv[n]; v.x *= r1; v.y *= r1; }
-        if (KIND == SK_GRAD2) { double r1 = a.rinv[n]; v.x *= r1; v.y *= r1; }
-      }
-      coef[(f * S_KC + kk) * S_NT + q] = v;
-    }
-    if (threadIdx.x < kc) spar[threadIdx.x] = a.hs[kbeg + k0 + threadIdx.x];
-    __syncthreads();
-    if (j < Th2) {
-      for (int kk = 0; kk < kc; ++kk) {
-        // parity is uniform across the block for a given k: branch so that every
-        // accumulator index is a compile-time constant (registers, no local memory)
-        if (spar[kk] == 0)
-          synth_accum<KIND, 0>(acc, tab, coef, kk, j, Th2);
-        else
-          synth_accum<KIND, 1>(acc, tab, coef, kk, j, Th2);
-      }
-    }
-  }
-  if (j >= Th2) return;
-#pragma unroll
-  for (int o = 0; o < NOUT; ++o)
-#pragma unroll
-    for (int q = 0; q < S_NT; ++q) {
-      int n = n0 + q;
-      if (n >= a.N) continue;
-      G.out[o][four_off(n, c, 0, j, a.NM, a.HB)] = acc[o][0][q];  // E
-      G.out[o][four_off(n, c, 1, j, a.NM, a.HB)] = acc[o][1][q];  // O
-    }
-}
-
-struct AnalArgs {
-  int N, H, Th, Th2, NM, HB, Hr, ngroup;
-  const int* perm;     // [Hc][Hr]: thread -> harmonic of the column, sorted by (m-counter, parity)
-  const int* mstart;   // per m-counter
-  const int* mlen;
-  const int* hs;
   const int* hm;
-  const double* leg;
-  AnalGroup g[4];
+  const double* leg;   // 8 tables [t][H][Th2]
+  const double* rinv;  // 1/r per shell
+  LegClass k[LG_MAXCLASS];
 };
 
-template <int KIND>
-__global__ void __launch_bounds__(288) k_anal(AnalArgs a) {
-  constexpr int NF = (KIND == AK_VECTOR) ? 3 : 1;
-  constexpr int NTAB = (KIND == AK_VECTOR) ? 3 : 1;
-  extern __shared__ double smem[];
-  const int col = blockIdx.x;        // folded column: m-counters 2col, 2col+1
-  const int n0 = blockIdx.y * A_NT;
-  const AnalGroup& G = a.g[blockIdx.z];
-  const int Th = a.Th, Th2 = a.Th2, Hr = a.Hr;
-  const int c0 = 2 * col, c1 = 2 * col + 1;
-  const int len0 = a.mlen[c0];
-  const int kbeg = a.mstart[c0];     // the column's harmonics are contiguous
-  double* tab = smem;                                         // [NTAB][A_JC][Hr]
-  double2* dat = (double2*)(smem + NTAB * A_JC * Hr);         // [2 cnt][NF][2 par][A_JC*A_NT + 1]
-  // threads are ordered by (m-counter, parity) so that a warp reads one data row (a smem
-  // broadcast); rows are padded by one element so that neighbouring rows use other banks
-  const bool active = threadIdx.x < Hr;
-  const int k = active ? a.perm[(size_t)col * Hr + threadIdx.x] : 0;
-  const int cl = (k < len0) ? 0 : 1;
-  const int s = active ? a.hs[kbeg + k] : 0;
-  double2 acc[NF][A_NT];
-#pragma unroll
-  for (int f = 0; f < NF; ++f)
-#pragma unroll
-    for (int q = 0; q < A_NT; ++q) acc[f][q] = make_double2(0.0, 0.0);
-  const int tabid[3] = {LSD_LEG_GWP, LSD_LEG_GWLLP_, LSD_LEG_GWLLSIN1MP};
+__device__ __forceinline__ uint32_t lg_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// asynchronous copies of 16 / 8 bytes; valid = false writes zeros and reads nothing
+__device__ __forceinline__ void cp16(void* dst, const void* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(lg_smem(dst)), "l"(src), "r"(valid ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp8(void* dst, const void* src, bool valid) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(lg_smem(dst)), "l"(src), "r"(valid ? 8 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
 
-  for (int j0 = 0; j0 < Th2; j0 += A_JC) {
-    const int jc = min(A_JC, Th2 - j0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < NTAB * jc * Hr; i += blockDim.x) {
-      int t = i / (jc * Hr), rem = i % (jc * Hr), kk = rem / jc, jj = rem % jc;
-      tab[(t * A_JC + jj) * Hr + kk] = a.leg[(size_t)tabid[t] * a.H * Th2 + (size_t)(kbeg + kk) * Th2 + j0 + jj];
-    }
-    for (int i = threadIdx.x; i < 2 * NF * A_NT * jc; i += blockDim.x) {
-      int jj = i % jc, rem = i / jc, q = rem % A_NT, rem2 = rem / A_NT, f = rem2 % NF, cc = rem2 / NF;
-      int n = n0 + q;
-      double2 e = make_double2(0.0, 0.0), o = e;
-      if (n < a.N) {  // folded E/O data (the FFT stage folded the two hemispheres)
-        const int cn = cc ? c1 : c0, j = j0 + jj;
-        e = G.in[f][four_off_a(n, cn, 0, j, a.N, Th2)];
-        o = G.in[f][four_off_a(n, cn, 1, j, a.N, Th2)];
+template <bool ANAL, bool VEC>
+__device__ __forceinline__ void leg_tile(const LegArgs& a, const LegClass& k, double* sm) {
+  constexpr int NTAB = VEC ? 2 : 1, SH = VEC ? 16 : 32;  // shells of a CTA's 64 columns
+  constexpr int TAB = ANAL ? LG_TAB_A : LG_TAB_S, STAGE = LG_DATA + 2 * TAB;
+  const int c = blockIdx.x / a.mtiles, m0 = (blockIdx.x - c * a.mtiles) * LG_BM;
+  const int nsh = k.ng * a.N, s0 = blockIdx.y * SH;
+  const int kbeg = a.mstart[c], klen = a.mlen[c], Th2 = a.Th2;
+  if (s0 >= nsh || (ANAL && 2 * m0 >= klen)) return;
+  const int tid = threadIdx.x, lane = tid & 31, par = tid >> 6, half = (tid >> 5) & 1;
+  const int lk = lane & 3, lq = lane >> 2;
+  // M rows of this warp: theta rows m0 .. (synthesis), harmonics par + 2 (m0 ..) (analysis)
+  const int mrows = ANAL ? (klen + 1 - par) / 2 - m0 : Th2 - m0;
+  const int klast = ANAL ? 2 * Th2 : klen;  // staged values per (shell, field) row
+  const int nch = (klast + 15) / 16;
+
+  // this thread copies value e of every chunk of the staged rows r0 + 8 i
+  const int e = tid & 15;
+  const cplx* src[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = (tid >> 4) + 8 * i, s = s0 + (VEC ? row >> 1 : row), f = VEC ? row & 1 : 0;
+    const int g = s / a.N, n = s - g * a.N;
+    src[i] = s < nsh ? k.in[f][g] + (ANAL ? four_off_a(n, c, 0, 0, a.N, Th2) : (size_t)n * a.H + kbeg) + e : nullptr;
+  }
+  const bool even = (Th2 & 1) == 0;
+  auto issue = [&](int ch) {
+    if (ch < nch) {
+      double* st = sm + (ch % LG_STAGES) * STAGE;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const bool ok = src[i] && ch * 16 + e < klast;
+        cp16(st + 2 * (((tid >> 4) + 8 * i) * LG_DROW + e), ok ? (const void*)(src[i] + ch * 16) : (const void*)a.leg, ok);
       }
-      dat[((cc * NF + f) * 2 + 0) * DROW + jj * A_NT + q] = e;
-      dat[((cc * NF + f) * 2 + 1) * DROW + jj * A_NT + q] = o;
+      double* tb = st + LG_DATA;
+      // table rows: kk x 48 theta (synthesis), harmonic x 8 theta (analysis)
+      auto rows = [&](auto cp, int W) {
+        const int per = (ANAL ? 8 : LG_BM) / W, nrow = ANAL ? 2 * LG_BM : 16;
+        for (int i = tid; i < NTAB * nrow * per; i += LG_THREADS) {
+          const int u = i % per, r = (i / per) % nrow, t = i / (per * nrow);
+          const int kk = ANAL ? 2 * m0 + r : ch * 16 + r, j = (ANAL ? ch * 8 : m0) + W * u;
+          const bool ok = kk < klen && j < Th2;
+          const double* p = ok ? a.leg + ((size_t)k.tab[t] * a.H + kbeg + kk) * Th2 + j : a.leg;
+          cp(tb + t * TAB + r * (ANAL ? LG_AA : LG_AS) + W * u, p, ok);
+        }
+      };
+      if (even) rows([](double* d, const double* p, bool ok) { cp16(d, p, ok); }, 2);
+      else rows([](double* d, const double* p, bool ok) { cp8(d, p, ok); }, 1);
     }
-    __syncthreads();
-    if (active) {
-      for (int jj = 0; jj < jc; ++jj) {
-        if (KIND == AK_VECTOR) {
-          const double gP = tab[(0 * A_JC + jj) * Hr + k];
-          const double A1 = tab[(1 * A_JC + jj) * Hr + k];
-          const double A2 = tab[(2 * A_JC + jj) * Hr + k];
-          const double2* Yr_s = dat + ((cl * NF + 0) * 2 + s) * DROW + jj * A_NT;
-          const double2* Yt_s = dat + ((cl * NF + 1) * 2 + s) * DROW + jj * A_NT;
-          const double2* Yt_o = dat + ((cl * NF + 1) * 2 + (1 - s)) * DROW + jj * A_NT;
-          const double2* Yp_s = dat + ((cl * NF + 2) * 2 + s) * DROW + jj * A_NT;
-          const double2* Yp_o = dat + ((cl * NF + 2) * 2 + (1 - s)) * DROW + jj * A_NT;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  double acc[LG_MT][LG_NT][2];
 #pragma unroll
-          for (int q = 0; q < A_NT; ++q) {
-            const double2 yr = Yr_s[q], yts = Yt_s[q], yto = Yt_o[q], yps = Yp_s[q], ypo = Yp_o[q];
-            acc[0][q].x += yr.x * gP;
-            acc[0][q].y += yr.y * gP;
-            acc[1][q].x += yto.x * A1 + yps.y * A2;
-            acc[1][q].y += yto.y * A1 - yps.x * A2;
-            acc[2][q].x += ypo.x * A1 - yts.y * A2;
-            acc[2][q].y += ypo.y * A1 + yts.x * A2;
+  for (int i = 0; i < LG_MT; ++i)
+#pragma unroll
+    for (int j = 0; j < LG_NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+
+  for (int i = 0; i < LG_STAGES - 1; ++i) issue(i);
+  for (int ch = 0; ch < nch; ++ch) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(LG_STAGES - 2) : "memory");
+    __syncthreads();  // chunk ch has landed for every thread; chunk ch - 1's stage is free
+    issue(ch + LG_STAGES - 1);
+    const double* st = sm + (ch % LG_STAGES) * STAGE;
+#pragma unroll
+    for (int seg = 0; seg < NTAB; ++seg) {
+      const int dp = VEC && seg == 0 ? 1 - par : par;  // parity of the data of this segment
+      const double* tb = st + LG_DATA + seg * TAB;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {  // four K each
+        const int ki = dp + 2 * (4 * q + lk);
+        double b[LG_NT];
+#pragma unroll
+        for (int j = 0; j < LG_NT; ++j) {
+          const int col = half * 32 + j * 8 + lq;
+          if (VEC) {  // columns: Re, Im of out0, Re, Im of out1 of a shell
+            const int comp = col & 3, f = seg ? 1 - (comp >> 1) : comp >> 1, part = seg ? 1 - (comp & 1) : comp & 1;
+            const double x = st[2 * (((col >> 2) * 2 + f) * LG_DROW + ki) + part];
+            b[j] = seg && (comp == 1 || comp == 2) ? -x : x;
+          } else {
+            b[j] = st[2 * ((col >> 1) * LG_DROW + ki) + (col & 1)];
           }
-        } else {
-          const double gP = tab[jj * Hr + k];
-          const double2* Y = dat + ((cl * NF + 0) * 2 + s) * DROW + jj * A_NT;
+        }
 #pragma unroll
-          for (int q = 0; q < A_NT; ++q) {
-            acc[0][q].x += Y[q].x * gP;
-            acc[0][q].y += Y[q].y * gP;
+        for (int i = 0; i < LG_MT; ++i) {
+          if (i * 8 < mrows) {
+            const double av = ANAL ? tb[(par + 2 * (i * 8 + lq)) * LG_AA + 4 * q + lk] : tb[ki * LG_AS + i * 8 + lq];
+#pragma unroll
+            for (int j = 0; j < LG_NT; ++j) dmma(acc[i][j], av, b[j]);
           }
         }
       }
     }
   }
-  if (!active) return;
-  const int nh = kbeg + k;
-  const bool m0 = a.hm[nh] == 0;
+
+  // accumulators: M row lq, columns 2 lk, 2 lk + 1 (Re, Im) of each tile
 #pragma unroll
-  for (int q = 0; q < A_NT; ++q) {
-    int n = n0 + q;
-    if (n >= a.N) continue;
-    size_t id = (size_t)n * a.H + nh;
-    if (KIND == AK_VECTOR) {
-      G.out[0][id] = acc[0][q];  // q%Im of m = 0 is kept (transform.fftw3.F90:869)
-      G.out[1][id] = make_double2(acc[1][q].x, m0 ? 0.0 : acc[1][q].y);
-      G.out[2][id] = make_double2(acc[2][q].x, m0 ? 0.0 : acc[2][q].y);
+  for (int j = 0; j < LG_NT; ++j) {
+    const int col = half * 32 + j * 8 + 2 * lk, s = s0 + (VEC ? col >> 2 : col >> 1);
+    if (s >= nsh) continue;
+    const int g = s / a.N, n = s - g * a.N;
+    cplx* out = k.out[VEC ? (col >> 1) & 1 : 0][g];
+    if (ANAL) {
+      out += (size_t)n * a.H + kbeg + par;
+      const bool zero = ((k.zero >> g) & 1) && a.hm[kbeg] == 0;
+#pragma unroll
+      for (int i = 0; i < LG_MT; ++i)
+        if (i * 8 + lq < mrows) out[2 * (m0 + i * 8 + lq)] = make_double2(acc[i][j][0], zero ? 0.0 : acc[i][j][1]);
     } else {
-      G.out[0][id] = make_double2(acc[0][q].x, m0 ? 0.0 : acc[0][q].y);
+      const int po = k.flip ? 1 - par : par;
+      const double f = k.scale ? a.rinv[n] : 1.0;
+#pragma unroll
+      for (int i = 0; i < LG_MT; ++i)
+        if (i * 8 + lq < mrows) {
+          const double x = acc[i][j][0] * f, y = acc[i][j][1] * f;
+          out[four_off(n, c, po, m0 + i * 8 + lq, a.NM, a.HB)] = k.rot ? make_double2(-y, x) : make_double2(x, y);
+        }
     }
   }
 }
 
-template <int KIND>
-int launch_synth_kind(lsd_ctx* ctx, const SynthGroup* groups, int ngroups) {
-  SynthArgs a;
-  a.N = ctx->N; a.H = ctx->H; a.Th = ctx->Th; a.Th2 = ctx->Th2; a.NM = ctx->NM; a.HB = ctx->HB;
-  a.mstart = ctx->d_mstart; a.mlen = ctx->d_mlen; a.hs = ctx->d_s; a.leg = ctx->d_leg;
-  a.rinv = ctx->d_rinv;
-  int ng = 0;
-  for (int i = 0; i < ngroups; ++i)
-    if (groups[i].kind == KIND) a.g[ng++] = groups[i];
-  if (ng == 0) return LSD_OK;
-  a.ngroup = ng;
-  constexpr int NIN = SK<KIND>::nin, NTAB = SK<KIND>::ntab;
-  size_t smem = sizeof(double) * NTAB * S_KC * ctx->Th2 + sizeof(double2) * NIN * S_KC * S_NT;
-  cudaFuncSetAttribute(k_synth<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_synth<KIND>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  int threads = ((ctx->Th2 + 31) / 32) * 32;
-  dim3 grid(ctx->NM, ceil_div(ctx->N, S_NT), ng);
-  k_synth<KIND><<<grid, threads, smem, ctx->stream>>>(a);
-  ctx->launches++;
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return lsd_fail(ctx, LSD_ECUDA, std::string("k_synth: ") + cudaGetErrorString(e));
-  return LSD_OK;
+// grid (counters x M tiles, column blocks of the largest class, classes)
+template <bool ANAL>
+__global__ void __launch_bounds__(LG_THREADS, 3) k_leg(LegArgs a) {
+  extern __shared__ __align__(16) double lg_sm[];
+  const LegClass& k = a.k[blockIdx.z];
+  if (k.vec) leg_tile<ANAL, true>(a, k, lg_sm);
+  else leg_tile<ANAL, false>(a, k, lg_sm);
 }
 
-template <int KIND>
-int launch_anal_kind(lsd_ctx* ctx, const AnalGroup* groups, int ngroups) {
-  AnalArgs a;
-  a.N = ctx->N; a.H = ctx->H; a.Th = ctx->Th; a.Th2 = ctx->Th2; a.NM = ctx->NM; a.HB = ctx->HB; a.Hr = ctx->Hr;
-  a.mstart = ctx->d_mstart; a.mlen = ctx->d_mlen; a.hs = ctx->d_s; a.hm = ctx->d_m; a.leg = ctx->d_leg;
-  int ng = 0;
-  for (int i = 0; i < ngroups; ++i)
-    if (groups[i].kind == KIND) a.g[ng++] = groups[i];
-  if (ng == 0) return LSD_OK;
-  a.ngroup = ng;
-  constexpr int NF = (KIND == AK_VECTOR) ? 3 : 1;
-  size_t smem = sizeof(double) * NF * A_JC * ctx->Hr + sizeof(double2) * 2 * NF * 2 * DROW;
-  a.perm = ctx->d_aperm;
-  cudaFuncSetAttribute(k_anal<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_anal<KIND>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  int threads = ((ctx->Hr + 31) / 32) * 32;
-  if (threads > 1024) return lsd_fail(ctx, LSD_EARG, "analysis: folded column longer than 1024 harmonics");
-  dim3 grid(ctx->Hc, ceil_div(ctx->N, A_NT), ng);
-  k_anal<KIND><<<grid, threads, smem, ctx->stream>>>(a);
+// The classes of a launch: add() opens a class for its tables or joins the open one.
+struct LegBuilder {
+  LegArgs a{};
+  int nc = 0;
+  LegClass* find(int vec, int t1, int t2, int flip, int rot, int scale) {
+    for (int i = 0; i < nc; ++i) {
+      LegClass& k = a.k[i];
+      if (k.vec == vec && k.tab[0] == t1 && k.tab[1] == t2 && k.rot == rot && k.ng < LG_MAXG) return &k;
+    }
+    if (nc == LG_MAXCLASS) return nullptr;
+    LegClass& k = a.k[nc++];
+    k = LegClass{};
+    k.vec = vec; k.tab[0] = t1; k.tab[1] = t2; k.flip = flip; k.rot = rot; k.scale = scale;
+    return &k;
+  }
+  bool add(LegClass* k, const cplx* i0, const cplx* i1, cplx* o0, cplx* o1, bool zero) {
+    if (!k) return false;
+    k->in[0][k->ng] = i0; k->in[1][k->ng] = i1;
+    k->out[0][k->ng] = o0; k->out[1][k->ng] = o1;
+    if (zero) k->zero |= 1u << k->ng;
+    k->ng++;
+    return true;
+  }
+};
+
+template <bool ANAL>
+int launch_leg(lsd_ctx* ctx, LegBuilder& b) {
+  if (b.nc == 0) return LSD_OK;
+  LegArgs& a = b.a;
+  a.N = ctx->N; a.H = ctx->H; a.Th2 = ctx->Th2; a.NM = ctx->NM; a.HB = ctx->HB;
+  a.mstart = ctx->d_mstart; a.mlen = ctx->d_mlen; a.hm = ctx->d_m; a.leg = ctx->d_leg; a.rinv = ctx->d_rinv;
+  int klmax = 0, cols = 0;
+  for (int c = 0; c < ctx->NM; ++c) klmax = ctx->mlen[c] > klmax ? ctx->mlen[c] : klmax;
+  a.mtiles = ANAL ? ceil_div((klmax + 1) / 2, LG_BM) : ceil_div(ctx->Th2, LG_BM);
+  for (int i = 0; i < b.nc; ++i) {
+    const int n = ceil_div(a.k[i].ng * ctx->N, a.k[i].vec ? 16 : 32);
+    cols = n > cols ? n : cols;
+  }
+  const size_t smem = sizeof(double) * LG_STAGES * (LG_DATA + 2 * (ANAL ? LG_TAB_A : LG_TAB_S));
+  CUDA_TRY(cudaFuncSetAttribute(k_leg<ANAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k_leg<ANAL><<<dim3(ctx->NM * a.mtiles, cols, b.nc), LG_THREADS, smem, ctx->stream>>>(a);
   ctx->launches++;
   cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return lsd_fail(ctx, LSD_ECUDA, std::string("k_anal: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) return lsd_fail(ctx, LSD_ECUDA, std::string("k_leg: ") + cudaGetErrorString(e));
   return LSD_OK;
 }
 
@@ -341,18 +263,41 @@ int launch_anal_kind(lsd_ctx* ctx, const AnalGroup* groups, int ngroups) {
 
 int lsd_launch_synth(lsd_ctx* ctx, const SynthGroup* groups, int ngroups) {
   if (ctx->oz) return lsd_ozaki_launch_synth(ctx, groups, ngroups);  // LSD_PREC_OZAKI
-  int rc;
-  if ((rc = launch_synth_kind<SK_VECTOR>(ctx, groups, ngroups))) return rc;
-  if ((rc = launch_synth_kind<SK_SCALAR>(ctx, groups, ngroups))) return rc;
-  if ((rc = launch_synth_kind<SK_GRAD3>(ctx, groups, ngroups))) return rc;
-  if ((rc = launch_synth_kind<SK_GRAD2>(ctx, groups, ngroups))) return rc;
-  return LSD_OK;
+  LegBuilder b;
+  bool ok = true;
+  auto scalar = [&](const cplx* in, cplx* out, int tab, int flip, int rot, int scale) {
+    ok = ok && b.add(b.find(0, tab, -1, flip, rot, scale), in, nullptr, out, nullptr, false);
+  };
+  for (int i = 0; i < ngroups; ++i) {
+    const SynthGroup& G = groups[i];
+    if (G.kind == SK_VECTOR) {
+      scalar(G.in[0], G.out[0], LSD_LEG_P, 0, 0, 0);
+      ok = ok && b.add(b.find(1, LSD_LEG_LLP_, LSD_LEG_LLSIN1MP, 0, 0, 0), G.in[1], G.in[2], G.out[1], G.out[2], false);
+    } else if (G.kind == SK_SCALAR) {
+      scalar(G.in[0], G.out[0], LSD_LEG_P, 0, 0, 0);
+    } else {  // gradients: (C/r) dP/dtheta, i (C/r) m P / sin(theta)
+      const bool three = G.kind == SK_GRAD3;
+      if (three) scalar(G.in[0], G.out[0], LSD_LEG_P, 0, 0, 0);
+      scalar(G.in[three ? 1 : 0], G.out[three ? 1 : 0], LSD_LEG_P_, 1, 0, 1);
+      scalar(G.in[three ? 1 : 0], G.out[three ? 2 : 1], LSD_LEG_SIN1MP, 0, 1, 1);
+    }
+  }
+  if (!ok) return lsd_fail(ctx, LSD_EARG, "synthesis: too many groups in one launch");
+  return launch_leg<false>(ctx, b);
 }
 
 int lsd_launch_anal(lsd_ctx* ctx, const AnalGroup* groups, int ngroups) {
   if (ctx->oz) return lsd_ozaki_launch_anal(ctx, groups, ngroups);  // LSD_PREC_OZAKI
-  int rc;
-  if ((rc = launch_anal_kind<AK_VECTOR>(ctx, groups, ngroups))) return rc;
-  if ((rc = launch_anal_kind<AK_SCALAR>(ctx, groups, ngroups))) return rc;
-  return LSD_OK;
+  if (ceil_div(ctx->Hr, 32) * 32 > 1024) return lsd_fail(ctx, LSD_EARG, "analysis: folded column longer than 1024 harmonics");
+  LegBuilder b;
+  bool ok = true;
+  for (int i = 0; i < ngroups; ++i) {
+    const AnalGroup& G = groups[i];
+    const bool vec = G.kind == AK_VECTOR;  // q keeps Im of m = 0 (transform.fftw3.F90:869)
+    ok = ok && b.add(b.find(0, LSD_LEG_GWP, -1, 0, 0, 0), G.in[0], nullptr, G.out[0], nullptr, !vec);
+    if (vec)
+      ok = ok && b.add(b.find(1, LSD_LEG_GWLLP_, LSD_LEG_GWLLSIN1MP, 0, 0, 0), G.in[1], G.in[2], G.out[1], G.out[2], true);
+  }
+  if (!ok) return lsd_fail(ctx, LSD_EARG, "analysis: too many groups in one launch");
+  return launch_leg<true>(ctx, b);
 }
