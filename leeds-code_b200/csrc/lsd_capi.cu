@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "lsd_common.cuh"
+#include "lsd_stream.cuh"
 
 static_assert(sizeof(PcState) == sizeof(lsd_pc_state), "lsd_pc_state mirrors PcState");
 
@@ -40,12 +41,12 @@ void free_ctx(lsd_ctx* ctx) {
   lsd_ozaki_free(ctx);
   void* ptrs[] = {ctx->d_l, ctx->d_m, ctx->d_s, ctx->d_mc, ctx->d_mstart, ctx->d_mlen, ctx->d_thm, ctx->d_bin2c, ctx->d_lm2nh,
                   ctx->d_leg, ctx->d_gp, ctx->d_gw, ctx->d_sn, ctx->d_sn1, ctx->d_tw2, ctx->d_twh, ctx->d_r,
-                  ctx->d_dr, ctx->d_r1dr, ctx->d_radlap, ctx->d_intr2dr, ctx->d_lu, ctx->d_lus, ctx->d_y, ctx->d_yt,
-                  ctx->d_ipiv, ctx->d_ipivs, ctx->d_info, ctx->d_gre, ctx->d_gret, ctx->d_invg, ctx->d_state, ctx->d_nl,
+                  ctx->d_dr, ctx->d_r1dr, ctx->d_radlap, ctx->d_intr2dr, ctx->d_lu, ctx->d_y, ctx->d_lf, ctx->d_uf, ctx->d_yf,
+                  ctx->d_ipiv, ctx->d_info, ctx->d_gf, ctx->d_invg, ctx->d_state, ctx->d_nl,
                   ctx->d_sv, ctx->d_spec, ctx->d_four, ctx->d_phys, ctx->d_red, ctx->d_cpart, ctx->d_ref, ctx->d_laps,
                   ctx->d_compr1dr, ctx->d_wts, ctx->d_ones, ctx->d_cfl, ctx->d_icr, ctx->d_icdr, ctx->d_icradlap,
                   ctx->d_icr1dr, ctx->d_icintr2dr, ctx->d_icwts, ctx->d_icref, ctx->d_iclaps, ctx->d_iccompr1dr,
-                  ctx->d_icyt, ctx->d_icstate, ctx->d_icsv, ctx->d_rot, ctx->d_gwP0, ctx->d_grescr,
+                  ctx->d_icyf, ctx->d_icstate, ctx->d_icsv, ctx->d_rot, ctx->d_gwP0, ctx->d_grescr,
                   ctx->d_pc, ctx->d_opfail};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -639,11 +640,20 @@ int lsd_create(const lsd_config* cfg, lsd_ctx** out) {
     if (ctx->hl[nh] == 1 && ctx->hm[nh] == 1) ctx->nh_l1m1 = nh;
   }
   const int NL = ctx->NL;
-  const size_t lus = (size_t)OP_NFAM * L * NL * (3 * KL + 1);
-  TRY(dalloc(ctx, &ctx->d_lu, lus)); TRY(dalloc(ctx, &ctx->d_lus, lus));
+  // the solve layouts keep zeros in their padding rows and lanes
+  const int nlb = ctx->nlb = ceil_div(L, 32);
+  auto zalloc = [&](double** p, size_t n) {
+    int r = dalloc(ctx, p, n);
+    if (!r && cudaMemsetAsync(*p, 0, sizeof(double) * n, ctx->stream) != cudaSuccess) r = LSD_ECUDA;
+    return r;
+  };
+  const size_t lanes = (size_t)nlb * 32, rNL = sv_rows(NL, KL), rN = sv_rows(N, KL);
+  TRY(dalloc(ctx, &ctx->d_lu, (size_t)OP_NFAM * L * NL * (3 * KL + 1)));
   TRY(dalloc(ctx, &ctx->d_y, (size_t)OP_NFAM * N * (2 * KL + 1) * L));
-  TRY(dalloc(ctx, &ctx->d_yt, (size_t)OP_NFAM * N * (2 * KL + 1) * L));
-  TRY(dalloc(ctx, &ctx->d_ipiv, (size_t)OP_NFAM * L * NL)); TRY(dalloc(ctx, &ctx->d_ipivs, (size_t)OP_NFAM * L * NL));
+  TRY(dalloc(ctx, &ctx->d_ipiv, (size_t)OP_NFAM * L * NL));
+  TRY(zalloc(&ctx->d_lf, (OP_NFAM + 1) * lanes * rNL * (KL + 1)));
+  TRY(zalloc(&ctx->d_uf, OP_NFAM * lanes * rNL * (2 * KL + 2)));
+  TRY(zalloc(&ctx->d_yf, OP_NFAM * lanes * rN * (2 * KL + 1)));
   if (ctx->Nic > 1) {  // the inner core's mesh, field, saved terms and Y bands
     const int Ni = ctx->Nic;
     TRY(dalloc(ctx, &ctx->d_icr, (size_t)7 * Ni));
@@ -658,7 +668,7 @@ int lsd_create(const lsd_config* cfg, lsd_ctx** out) {
     std::vector<double> ref((size_t)7 * Ni, 0.0);
     for (int n = 0; n < Ni; ++n) ref[(size_t)REF_ETA * Ni + n] = 1.0;
     TRY(upload(ctx, ctx->d_icref, ref));
-    TRY(dalloc(ctx, &ctx->d_icyt, (size_t)2 * Ni * (2 * KL + 1) * L));
+    TRY(zalloc(&ctx->d_icyf, 2 * lanes * sv_rows(Ni, KL) * (2 * KL + 1)));
     TRY(dalloc(ctx, &ctx->d_icstate, (size_t)2 * Ni * H)); TRY(dalloc(ctx, &ctx->d_icsv, (size_t)2 * Ni * H));
     CTRY(cudaMemsetAsync(ctx->d_icstate, 0, sizeof(cplx) * 2 * Ni * H, ctx->stream));
     CTRY(cudaMemsetAsync(ctx->d_icsv, 0, sizeof(cplx) * 2 * Ni * H, ctx->stream));
@@ -671,9 +681,9 @@ int lsd_create(const lsd_config* cfg, lsd_ctx** out) {
     ctx->rot_inertia = (8.0 * 3.1415926535897931 / 15.0) * (r4 * ri);
   }
   TRY(dalloc(ctx, &ctx->d_info, (size_t)OP_NFAM * L));
-  TRY(dalloc(ctx, &ctx->d_gre, (size_t)L * 2 * N)); TRY(dalloc(ctx, &ctx->d_invg, (size_t)L * 4));
-  TRY(dalloc(ctx, &ctx->d_gret, (size_t)L * 2 * N));
-  TRY(dalloc(ctx, &ctx->d_grescr, (size_t)L * N));
+  TRY(dalloc(ctx, &ctx->d_invg, (size_t)L * 4));
+  TRY(zalloc(&ctx->d_gf, lanes * rN * 2));
+  TRY(dalloc(ctx, &ctx->d_grescr, lanes * N));
   const size_t F = (size_t)N * H;
   TRY(dalloc(ctx, &ctx->d_state, LSD_NFIELD * F)); TRY(dalloc(ctx, &ctx->d_nl, LSD_NFIELD * F));
   TRY(dalloc(ctx, &ctx->d_sv, LSD_NFIELD * F));
@@ -693,7 +703,7 @@ int lsd_create(const lsd_config* cfg, lsd_ctx** out) {
   }
   TRY(dalloc(ctx, &ctx->d_four, (size_t)ctx->nfour * N * ctx->HB * NM * 4));
   TRY(dalloc(ctx, &ctx->d_red, (size_t)128 + 48 * N));
-  TRY(dalloc(ctx, &ctx->d_cpart, (size_t)8 * ((H + 31) / 32)));
+  TRY(dalloc(ctx, &ctx->d_cpart, (size_t)8 * nlb * c.M));
   TRY(dalloc(ctx, &ctx->d_cfl, (size_t)2 * N + 1));
   CTRY(cudaMallocHost((void**)&ctx->h_red, sizeof(double) * 64));
   // pinned staging: three spectral fields, and at least the host staging of the energy

@@ -135,24 +135,25 @@ struct lsd_ctx {
   // conducting inner core (Nic > 1): its mesh (the same tables as the outer core's on
   // Nic points: r powers [7][Nic], dr bands, radLap, r1dr, intr2dr, weighted weights,
   // reference columns [7][Nic] with eta = 1, reference bands, compr1dr); its field
-  // [2][Nic][H] (mag_icTor, mag_icPol) and saved nonlinear terms; the Y bands of its two
-  // families [2][Nic][2KL+1][L].  NL = N + Nic - 1 rows per operator (the field families'
+  // [2][Nic][H] (mag_icTor, mag_icPol) and saved nonlinear terms.  NL = N + Nic - 1 rows per operator (the field families'
   // coupled systems; N rows used by the others).
   int Nic = 1, NL = 0;
   double *d_icr = nullptr, *d_icdr = nullptr, *d_icradlap = nullptr, *d_icr1dr = nullptr, *d_icintr2dr = nullptr;
-  double *d_icwts = nullptr, *d_icref = nullptr, *d_iclaps = nullptr, *d_iccompr1dr = nullptr, *d_icyt = nullptr;
+  double *d_icwts = nullptr, *d_icref = nullptr, *d_iclaps = nullptr, *d_iccompr1dr = nullptr;
   cplx *d_icstate = nullptr, *d_icsv = nullptr;
   // inner-core rotation (rotation.F90), ROT_* slots; Gauss weight x P_0^0 / 2 per theta
   double *d_rot = nullptr, *d_gwP0 = nullptr;
   double rot_inertia = 0.0;
-  // operators: LAPACK band LU [fam][L][N][3KL+1] + ipiv [fam][L][N]; Y bands
-  // [fam][L][N][2KL+1]; (d_lus / d_ipivs: [fam][N][3KL+1][L] copies, l fastest)
-  double *d_lu = nullptr, *d_lus = nullptr, *d_y = nullptr, *d_yt = nullptr;
-  int *d_ipiv = nullptr, *d_ipivs = nullptr, *d_info = nullptr;
-  double *d_gre = nullptr;   // [L][2][N]
-  double *d_gret = nullptr;  // [N][2][L]
+  // operators: LAPACK band LU [fam][L][NL][3KL+1] + ipiv [fam][L][NL]; Y bands
+  // [fam][L][N][2KL+1]; in the solve layouts (lsd_stream.cuh, nlb blocks of 32 degrees) the L
+  // rows (and a family of zeros), U rows, Y rows, the inner core's Y rows, and the poloidal
+  // velocity's Green's functions [nlb][N + pads][2][32]
+  int nlb = 0;
+  double *d_lu = nullptr, *d_y = nullptr, *d_lf = nullptr, *d_uf = nullptr, *d_yf = nullptr, *d_icyf = nullptr;
+  double *d_gf = nullptr;
+  int *d_ipiv = nullptr, *d_info = nullptr;
   double *d_invg = nullptr;  // [L][4]
-  double2 *d_grescr = nullptr;  // [N][L] scratch of k_greens
+  double2 *d_grescr = nullptr;  // [N][32 nlb] scratch of k_greens
   bool have_ops = false;
   double op_dt = 0.0;
   // state, nonlinear terms, saved nonlinear terms: [field][N][H] complex
@@ -171,7 +172,7 @@ struct lsd_ctx {
   size_t h_pin_bytes = 0;
   // reductions
   double *d_red = nullptr;   // small reduction area
-  double *d_cpart = nullptr; // corrector: per-warp sums of squares [8][ceil(H / 32)]
+  double *d_cpart = nullptr; // corrector: per-warp sums of squares [8][nlb][M]
   double *h_red = nullptr;   // pinned mirror (64 doubles; slots below)
   // time
   double t = 0.0, dt = 0.0, dterr = 0.0, corr_dt = 0.0, lasterr = 1e99, cfl_dt = 0.0;

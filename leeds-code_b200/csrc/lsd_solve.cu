@@ -12,6 +12,7 @@
 #include <cstdio>
 
 #include "lsd_common.cuh"
+#include "lsd_stream.cuh"
 
 namespace {
 
@@ -202,24 +203,18 @@ __global__ void k_tail(TailArgs a) {
 }
 
 // ---------------------------------------------------------------------------------------
-// Column solves.  A thread owns one harmonic nh of one field: its Re and Im columns
+// Column solves (lsd_stream.cuh).  A thread owns one harmonic of one field: its Re and Im columns
 // x(n) = X[n * H + nh] (complex), solved with the same factors like the reference's two
-// dgbtrs calls (tim_invX, timestep.F90:566-588).  Consecutive threads take consecutive
-// harmonics, so every row access of a warp is one contiguous 512-byte segment, and the
-// factors are read from copies with the degree l fastest ([fam][n][band][l]), so a
-// warp's factor reads are contiguous too.  Columns stream through register windows:
-// KL + 1 rows for the forward elimination with row interchanges, 2 KL + 1 for the banded
-// back substitution, right-hand-side rows fetched SPF rows ahead; intermediate columns
-// go to per-field scratch in global memory.
+// dgbtrs calls (tim_invX, timestep.F90:566-588).  CTA (block of 32 degrees, group of T / 32
+// orders); intermediate columns go to per-field scratch in global memory.
 // ---------------------------------------------------------------------------------------
 struct StepArgs {
-  int N, H, KL, L;
-  const int* hl;
-  const int* hm;
-  const double* lus;   // [fam][N][3KL+1][L] LAPACK band factors, l fastest
-  const int* ipivs;    // [fam][N][L]
-  const double* yt;    // [fam][N][2KL+1][L] Y bands, l fastest
-  const double* gret;  // [N][2][L] Green's functions
+  int N, H, L, nlb, M, Mp;
+  const int* mstart;   // per m-counter
+  const int* bin2c;    // order index -> m-counter
+  // factors in the solve layouts (lsd_stream.cuh): L rows (one more family of zeros), U rows (NL
+  // rows a family), Y rows (N), the Green's functions [nlb][N + pads][2][32]
+  const double *lf, *uf, *yf, *gf;
   const double* invg;  // [L][4]
   cplx* state;  // [field][N][H]
   cplx* nl;
@@ -229,23 +224,22 @@ struct StepArgs {
   int cod_bc, comp_bc, vel_bc;
   double qi, qo, qi_comp, qo_comp;
   int comp;
-  double* red;  // corrector: [8] sums of squares
   double* cpart;  // corrector: the per-warp sums [8][nwarp] that k_cgce_sums adds up
-  int nwarp;      // ceil(H / 32)
+  int nwarp;      // (blocks of 32 degrees) x orders
   int NL;       // rows per operator in lus / ipivs (N + Nic - 1)
   int Nic;      // inner-core points (> 1: conducting, the field families are coupled)
   cplx* icstate;       // [2][Nic][H] mag_icTor, mag_icPol
   cplx* icsv;          // [2][Nic][H] their saved nonlinear terms
-  const double* icyt;  // [2][Nic][2KL+1][L] the inner core's Y bands
+  const double* icyf;  // the inner core's Y rows (2 families of Nic rows)
   const double* rot;   // ROT_* slots: rot_omega and the rate of the last evaluation
   const double* rtor10;  // vel_setbc_Tor's mes_oc%r(1, nh) at nh of (l, m) = (1, 0)
 };
 
-// which solve a grid row performs
-enum SolveJob { J_VTOR = 0, J_VPOL, J_COD, J_MTOR, J_MPOL, J_COMP, J_NJOB };
+// which solve a grid row performs; the poloidal velocity's two solves are the longest chain and
+// come first
+enum SolveJob { J_VPOL = 0, J_MTOR, J_MPOL, J_VTOR, J_COD, J_COMP, J_NJOB };
 
 constexpr int SOLVE_THREADS = 128;
-constexpr int SPF = 8;  // right-hand-side rows fetched ahead, so that their loads overlap
 
 __device__ __forceinline__ int job_field(int job) {
   return job == J_VTOR ? LSD_VEL_TOR : job == J_VPOL ? LSD_VEL_POL : job == J_COD ? LSD_COD_C
@@ -256,307 +250,63 @@ __device__ __forceinline__ int job_family(int job) {
        : job == J_MTOR ? OP_MTOR : OP_MPOL;
 }
 
-// band factor element (row r 0-based, column c) of this thread's degree: f[(c LD + r) L]
-struct Band {
-  const double* f;
-  const int* piv;
-  int L, LD;
-  __device__ double at(int r, int c) const { return __ldg(f + ((size_t)c * LD + r) * L); }
-  __device__ int pivot(int c) const { return __ldg(piv + (size_t)c * L); }
+// The column of a thread: block of 32 degrees lb, order index mi (warp), degree l (lane).
+struct ColId {
+  int lb, mi, l, nh, warp;  // warp: lb M + mi, the slot of the corrector's partial sums
+  bool on;                  // (l, m) exists
 };
-
-__device__ __forceinline__ double2 axpy2(double2 y, double a, double2 x) {  // y + a x
-  return make_double2(y.x + a * x.x, y.y + a * x.y);
+__device__ __forceinline__ ColId col_id(int L, int M, int Mp, const int* mstart, const int* bin2c) {
+  const int groups = (M * 32 + blockDim.x - 1) / blockDim.x;
+  ColId c;
+  c.lb = blockIdx.x / groups;
+  c.mi = (blockIdx.x - c.lb * groups) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  c.l = c.lb * 32 + (threadIdx.x & 31);
+  c.on = c.mi < M && c.l < L && c.l >= c.mi * Mp;
+  c.nh = c.on ? mstart[bin2c[c.mi]] + c.l - c.mi * Mp : 0;
+  c.warp = c.mi < M ? c.lb * M + c.mi : -1;
+  return c;
+}
+// no warp of the CTA has a column: the block's degrees end below its first order
+__device__ __forceinline__ bool cta_empty(const ColId& c, int M, int Mp) {
+  const int m0 = c.mi - (threadIdx.x >> 5);
+  return m0 >= M || c.lb * 32 + 31 < m0 * Mp;
 }
 
-// dgbtrs forward part (LAPACK order): for c = 0..N-2 swap rows c and piv(c), then
-// x(c+i) -= L(c+i, c) x(c), i <= KL.  in(n) supplies right-hand-side rows in increasing
-// n (each once); out(c, y) receives the finished rows.  The right-hand-side rows and the
-// factors of a batch of SPF rows are loaded before its arithmetic.
-template <int KL, class IN, class OUT>
-__device__ __forceinline__ void stream_forward(const Band& B, int N, IN&& in, OUT&& out) {
-  constexpr int KD = 2 * KL + 1;
-  double2 w[KL + 1];
-#pragma unroll
-  for (int i = 0; i <= KL; ++i) w[i] = i < N ? in(i) : make_double2(0.0, 0.0);
-  for (int c0 = 0; c0 < N; c0 += SPF) {
-    double2 buf[SPF];  // rows c0 + KL + 1 + u, requested in increasing order
-    int pv[SPF];
-    double lf[SPF][KL];
-#pragma unroll
-    for (int u = 0; u < SPF; ++u) {
-      const int c = min(c0 + u, N - 1);
-      pv[u] = B.pivot(c);
-#pragma unroll
-      for (int i = 0; i < KL; ++i) lf[u][i] = B.at(KD + i, c);
-    }
-#pragma unroll
-    for (int u = 0; u < SPF; ++u) buf[u] = c0 + KL + 1 + u < N ? in(c0 + KL + 1 + u) : make_double2(0.0, 0.0);
-#pragma unroll
-    for (int u = 0; u < SPF; ++u) {
-      const int c = c0 + u;
-      if (c >= N) break;
-      if (c < N - 1) {
-        const int p = pv[u] - 1 - c;  // 0..KL
-#pragma unroll
-        for (int i = 1; i <= KL; ++i)
-          if (p == i) { const double2 t = w[0]; w[0] = w[i]; w[i] = t; }
-        const double2 temp = make_double2(-w[0].x, -w[0].y);
-#pragma unroll
-        for (int i = 1; i <= KL; ++i)
-          if (c + i < N) w[i] = axpy2(w[i], lf[u][i - 1], temp);
-      }
-      out(c, w[0]);
-#pragma unroll
-      for (int i = 0; i < KL; ++i) w[i] = w[i + 1];
-      w[KL] = buf[u];
-    }
-  }
-}
-
-// dtbsv (upper, non-unit, bandwidth 2KL; LAPACK column order) on the forward result:
-// for c = N-1..0: x(c) = y(c) / U(c, c); x(c-t) -= x(c) U(c-t, c), t <= 2KL.
-// in(n) supplies y rows in decreasing n; out(c, x) receives x(c) in decreasing c.
-constexpr int SPB = 8;  // rows per batch of the back substitution
-template <int KL, class IN, class OUT>
-__device__ __forceinline__ void stream_backward(const Band& B, int N, IN&& in, OUT&& out) {
-  constexpr int K2 = 2 * KL;
-  double2 w[K2 + 1];  // w[t] = pending y(c - t)
-#pragma unroll
-  for (int t = 0; t <= K2; ++t) w[t] = N - 1 - t >= 0 ? in(N - 1 - t) : make_double2(0.0, 0.0);
-  for (int c0 = N - 1; c0 >= 0; c0 -= SPB) {
-    double2 buf[SPB];  // rows c0 - K2 - 1 - u
-    double uf[SPB][K2 + 1];
-#pragma unroll
-    for (int u = 0; u < SPB; ++u) {
-      const int c = max(c0 - u, 0);
-#pragma unroll
-      for (int t = 0; t <= K2; ++t) uf[u][t] = B.at(K2 - t, c);  // uf[u][0] = U(c, c)
-    }
-#pragma unroll
-    for (int u = 0; u < SPB; ++u) buf[u] = c0 - K2 - 1 - u >= 0 ? in(c0 - K2 - 1 - u) : make_double2(0.0, 0.0);
-#pragma unroll
-    for (int u = 0; u < SPB; ++u) {
-      const int c = c0 - u;
-      if (c < 0) break;
-      const double d = uf[u][0];
-      const double2 xc = make_double2(w[0].x / d, w[0].y / d);
-      out(c, xc);
-      const double2 mx = make_double2(-xc.x, -xc.y);
-#pragma unroll
-      for (int t = 1; t <= K2; ++t) w[t] = axpy2(w[t], uf[u][t], mx);
-#pragma unroll
-      for (int t = 0; t < K2; ++t) w[t] = w[t + 1];
-      w[K2] = buf[u];
-    }
-  }
-}
-
-// W(n) := (Y X)(n) + R(n) with the Y band (2KL+1, N) for every row of a column (tim_multY,
-// timestep.F90:640-670) as a pass of its own, eight rows per batch: the batch's X rows,
-// band values and R rows are all loaded before any of its rows is stored, so their loads
-// overlap (a window advanced one row per streamed row would wait for each X row in turn).
-// R may be W (in place) or the nonlinear terms.  Only arrays that no thread of the kernel
-// writes (the bands, the nonlinear terms) go through the read-only path (__ldg): that path
-// lets the compiler move a load past a store to the same address.
-constexpr int MY_BATCH = 8;
-template <int KL>
-__device__ __forceinline__ void multy_rows(const double* y, int L, const double2* X, const double2* R, double2* W,
-                                           size_t rst, int N) {
-  constexpr int LDM = 2 * KL + 1, WIN = 2 * KL + MY_BATCH;
-  double2 win[WIN];  // X rows n0 - KL .. n0 + MY_BATCH - 1 + KL
-#pragma unroll
-  for (int t = 0; t < 2 * KL; ++t) {
-    const int j = t - KL;
-    win[t] = (j >= 0 && j < N) ? X[(size_t)j * rst] : make_double2(0.0, 0.0);
-  }
-  for (int n0 = 0; n0 < N; n0 += MY_BATCH) {
-    double2 r[MY_BATCH];
-    double yb[MY_BATCH][LDM];
-#pragma unroll
-    for (int u = 0; u < MY_BATCH; ++u) {
-      const int j = n0 + KL + u;
-      win[2 * KL + u] = j < N ? X[(size_t)j * rst] : make_double2(0.0, 0.0);
-      const int n = n0 + u;
-      r[u] = n < N ? R[(size_t)n * rst] : make_double2(0.0, 0.0);
-#pragma unroll
-      for (int t = 0; t < LDM; ++t) {
-        const int jj = n - KL + t;
-        yb[u][t] = (n < N && jj >= 0 && jj < N) ? __ldg(y + ((size_t)jj * LDM + (LDM - 1 - t)) * L) : 0.0;
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < MY_BATCH; ++u) {
-      double2 acc = r[u];
-#pragma unroll
-      for (int t = 0; t < LDM; ++t) acc = axpy2(acc, yb[u][t], win[u + t]);
-      if (n0 + u < N) W[(size_t)(n0 + u) * rst] = acc;
-    }
-#pragma unroll
-    for (int t = 0; t < 2 * KL; ++t) win[t] = win[t + MY_BATCH];
-  }
-}
-
-__device__ __forceinline__ void warp_partial(double v, const StepArgs& a, int slot);
-
-// per-thread view of one field's columns and this degree's operators
+// per-thread view of one field's columns
 struct ColView {
   double2 *X, *S, *W1, *W2;
   const double2* Nn;
-  size_t rst;
-  Band B1, B2;       // main operator; Green's operator (poloidal velocity)
-  const double* y1;  // Y band of the main family
-  const double* g;   // Green's functions: element (n, k) at g[(n 2 + k) L]
-  double iG[4];
 };
 
-template <int KL>
-__device__ ColView col_view(const StepArgs& a, int job, int nh, int l) {
+__device__ __forceinline__ ColView col_view(const StepArgs& a, int job, const ColId& c) {
   ColView v;
-  const int N = a.N, L = a.L, fam = job_family(job), fld = job_field(job);
-  constexpr int LD = 3 * KL + 1, LDM = 2 * KL + 1;
-  const size_t F = (size_t)N * a.H;
-  v.rst = a.H;
-  v.X = a.state + fld * F + nh;
-  v.Nn = a.nl + fld * F + nh;
-  v.S = a.sv + fld * F + nh;
-  v.W1 = a.work + (size_t)(2 * fld) * F + nh;
-  v.W2 = a.work + (size_t)(2 * fld + 1) * F + nh;
-  const int NL = a.NL;
-  v.B1.f = a.lus + (size_t)fam * NL * LD * L + l; v.B1.piv = a.ipivs + (size_t)fam * NL * L + l;
-  v.B1.L = L; v.B1.LD = LD;
-  v.B2.f = a.lus + (size_t)OP_VGRE * NL * LD * L + l; v.B2.piv = a.ipivs + (size_t)OP_VGRE * NL * L + l;
-  v.B2.L = L; v.B2.LD = LD;
-  v.y1 = a.yt + (size_t)fam * N * LDM * L + l;
-  v.g = a.gret + l;
-  for (int i = 0; i < 4; ++i) v.iG[i] = job == J_VPOL ? __ldg(a.invg + (size_t)l * 4 + i) : 0.0;
+  const int fld = job_field(job);
+  const size_t F = (size_t)a.N * a.H;
+  v.X = a.state + fld * F + c.nh;
+  v.Nn = a.nl + fld * F + c.nh;
+  v.S = a.sv + fld * F + c.nh;
+  v.W1 = a.work + (size_t)(2 * fld) * F + c.nh;
+  v.W2 = a.work + (size_t)(2 * fld + 1) * F + c.nh;
   return v;
 }
 
 // vel_gre_adjust (velocity.F90:445-465): coefficients of the two Green's functions
-__device__ __forceinline__ void gre_coeffs(const double* iG, double2 x0, double2 xN, double2& ca, double2& cb) {
+__device__ __forceinline__ void gre_coeffs(const double* invg, int l, double2 x0, double2 xN, double2& ca, double2& cb) {
+  double iG[4];
+  for (int i = 0; i < 4; ++i) iG[i] = __ldg(invg + (size_t)l * 4 + i);
   ca = make_double2(iG[0] * x0.x + iG[2] * xN.x, iG[0] * x0.y + iG[2] * xN.y);
   cb = make_double2(iG[1] * x0.x + iG[3] * xN.x, iG[1] * x0.y + iG[3] * xN.y);
 }
 
-// The saves of the nonlinear terms, apart from the streamed solves: every load of a batch of
-// eight rows is issued before its stores, so that a column's loads overlap.  (Inside the
-// streamed passes the right-hand-side callbacks only load: a store there would keep the
-// compiler from hoisting the next rows' loads above it, one memory round trip per row.)
-// save_terms: S := N.  diff_terms: W := c (N - S), S := N (tim_nlincorr).
-constexpr int SAVE_BATCH = 8;
-__device__ __forceinline__ void save_terms(const double2* Nn, double2* S, size_t rst, int N) {
-  for (int n0 = 0; n0 < N; n0 += SAVE_BATCH) {
-    double2 x[SAVE_BATCH];
-#pragma unroll
-    for (int u = 0; u < SAVE_BATCH; ++u)
-      if (n0 + u < N) x[u] = __ldg(Nn + (size_t)(n0 + u) * rst);
-#pragma unroll
-    for (int u = 0; u < SAVE_BATCH; ++u)
-      if (n0 + u < N) S[(size_t)(n0 + u) * rst] = x[u];
-  }
-}
-__device__ __forceinline__ void diff_terms(const double2* Nn, double2* S, double2* W, size_t rst, int N, double c) {
-  for (int n0 = 0; n0 < N; n0 += SAVE_BATCH) {
-    double2 x[SAVE_BATCH], p[SAVE_BATCH];
-#pragma unroll
-    for (int u = 0; u < SAVE_BATCH; ++u)
-      if (n0 + u < N) { x[u] = __ldg(Nn + (size_t)(n0 + u) * rst); p[u] = S[(size_t)(n0 + u) * rst]; }
-#pragma unroll
-    for (int u = 0; u < SAVE_BATCH; ++u)
-      if (n0 + u < N) {
-        S[(size_t)(n0 + u) * rst] = x[u];
-        W[(size_t)(n0 + u) * rst] = make_double2(c * (x[u].x - p[u].x), c * (x[u].y - p[u].y));
-      }
-  }
-}
-
-// Predictor (velocity.F90:369-395, codensity.F90:224-234, magnetic.F90:370-408).
-// grid (ceil(H / SOLVE_THREADS), J_NJOB).
-template <int KL>
-__global__ void __launch_bounds__(SOLVE_THREADS) k_predictor(StepArgs a) {
-  const int job = blockIdx.y;
-  if (job == J_COMP && !a.comp) return;
-  if ((job == J_MTOR || job == J_MPOL) && a.Nic > 1) return;  // k_mag_ic
-  const int nh = blockIdx.x * blockDim.x + threadIdx.x;
-  if (nh >= a.H) return;
-  const int l = a.hl[nh], N = a.N, L = a.L;
-  const bool zero = (job == J_COD || job == J_COMP);
-  const ColView v = col_view<KL>(a, job, nh, l);
-  const size_t rst = v.rst;
-  const double2 z2 = make_double2(0.0, 0.0);
-  // boundary rows of the right-hand side (tim_zerobc; cod_setbc / comp_setbc for l = 0)
-  double bc0 = 0.0, bcN = 0.0;
-  if (zero && nh == 0) {
-    const int bc = job == J_COD ? a.cod_bc : a.comp_bc;
-    const double qi = job == J_COD ? a.qi : a.qi_comp, qo = job == J_COD ? a.qo : a.qo_comp;
-    if (bc == 1 || bc == 2) bc0 = 1.0;
-    else if (bc == 3 || bc == 4) bc0 = qi;
-    bcN = (bc == 2 || bc == 4) ? qo : 0.0;
-  }
-  // vel_setbc_Tor (velocity.F90:291-300): the no-slip inner wall turns with the inner core
-  if (job == J_VTOR && l == 1 && a.hm[nh] == 0 && a.vel_bc <= 2) bc0 = a.rot[ROT_OMEGA] * a.rtor10[0];
-  auto w1 = [&](int c, double2 x) { v.W1[(size_t)c * rst] = x; };
-  auto r1 = [&](int n) { return v.W1[(size_t)n * rst]; };
-  if (job == J_VPOL) {
-    // Pol := NPol ; zerobc ; invX(XGre) ; Pol := YPol vel_Pol + Pol ; zerobc ; invX(XPol) ;
-    // vel_gre_adjust (velocity.F90:369-395, 445-465)
-    save_terms(v.Nn, v.S, rst, N);
-    auto inA = [&](int n) {
-      const double2 x = __ldg(v.Nn + (size_t)n * rst);
-      return (n == 0 || n == N - 1) ? z2 : x;
-    };
-    if (l == 0) {
-      for (int n = 0; n < N; ++n) v.X[(size_t)n * rst] = inA(n);
-      return;
-    }
-    stream_forward<KL>(v.B2, N, inA, w1);
-    stream_backward<KL>(v.B2, N, r1, [&](int c, double2 x) { v.W2[(size_t)c * rst] = x; });
-    multy_rows<KL>(v.y1, L, v.X, v.W2, v.W2, rst, N);  // YPol vel_Pol + Pol, in place
-    auto inB = [&](int n) { return (n == 0 || n == N - 1) ? z2 : v.W2[(size_t)n * rst]; };
-    double2 x0 = z2, xN = z2;
-    stream_forward<KL>(v.B1, N, inB, w1);
-    stream_backward<KL>(v.B1, N, r1, [&](int c, double2 x) {
-      v.W2[(size_t)c * rst] = x;
-      if (c == N - 1) xN = x;
-      if (c == 0) x0 = x;
-    });
-    double2 ca, cb;
-    gre_coeffs(v.iG, x0, xN, ca, cb);
-#pragma unroll 8
-    for (int n = 0; n < N; ++n) {
-      const double g1 = __ldg(v.g + (size_t)(2 * n) * L), g2 = __ldg(v.g + (size_t)(2 * n + 1) * L);
-      const double2 x = v.W2[(size_t)n * rst];
-      v.X[(size_t)n * rst] = make_double2(x.x - ca.x * g1 - cb.x * g2, x.y - ca.y * g1 - cb.y * g2);
-    }
-    return;
-  }
-  // other fields: X := Y X + N ; zerobc (+ setbc) ; invX
-  const bool solve = (l != 0 || zero);
-  save_terms(v.Nn, v.S, rst, N);
-  if (!solve) {
-    for (int n = 0; n < N; ++n)
-      v.X[(size_t)n * rst] = n == 0 ? make_double2(bc0, 0.0) : n == N - 1 ? make_double2(bcN, 0.0)
-                                                                         : __ldg(v.Nn + (size_t)n * rst);
-    return;
-  }
-  multy_rows<KL>(v.y1, L, v.X, v.Nn, v.W1, rst, N);  // Y X + N into W1 (solved in place)
-  auto inC = [&](int n) {
-    if (n == 0) return make_double2(bc0, 0.0);
-    if (n == N - 1) return make_double2(bcN, 0.0);
-    return v.W1[(size_t)n * rst];
-  };
-  stream_forward<KL>(v.B1, N, inC, w1);
-  stream_backward<KL>(v.B1, N, r1, [&](int c, double2 x) { v.X[(size_t)c * rst] = x; });
-}
-
-// the warp's sum of v (harmonics 32 w .. 32 w + 31) into its own slot of the corrector's
-// partials: the sums reach k_cgce_sums in a fixed order, so the corrector norm -- and the
-// timestep the norm controls -- are the same bits on every run
-__device__ __forceinline__ void warp_partial(double v, const StepArgs& a, int slot) {
+// the warp's sum of v into its own slot of the corrector's partials: the sums reach k_cgce_sums
+// in a fixed order, so the corrector norm -- and the timestep the norm controls -- are the same
+// bits on every run
+__device__ __forceinline__ void warp_partial(double v, const StepArgs& a, int slot, int warp) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if ((threadIdx.x & 31) == 0 && w < a.nwarp) a.cpart[(size_t)slot * a.nwarp + w] = v;  // w >= nwarp: no harmonic
+  if ((threadIdx.x & 31) == 0 && warp >= 0) a.cpart[(size_t)slot * a.nwarp + warp] = v;
+}
+__device__ __forceinline__ int job_slot(int job) {
+  return job == J_VTOR ? 0 : job == J_VPOL ? 1 : job == J_COD ? 2 : job == J_COMP ? 3 : job == J_MTOR ? 4 : 6;
 }
 
 // red[s] = the sum of the per-warp partials of slot s; one warp per slot, lanes over the
@@ -569,174 +319,173 @@ __global__ void k_cgce_sums(const double* part, int nwarp, double* red) {
   if (lane == 0) red[s] = v;
 }
 
-// Corrector (velocity.F90:413-439, codensity.F90:240-259, magnetic.F90:414-461)
-// red[] slots: 0 vTor, 1 vPol, 2 cod, 3 comp, 4 bTor, 5 bicTor, 6 bPol, 7 bicPol.
-// The sum of squares of the corrections is accumulated per harmonic in the order the
-// back substitution produces them (n decreasing) and across harmonics by atomics.
-template <int KL>
-__global__ void __launch_bounds__(SOLVE_THREADS) k_corrector(StepArgs a) {
-  const int job = blockIdx.y;
-  if (job == J_COMP && !a.comp) return;
-  if ((job == J_MTOR || job == J_MPOL) && a.Nic > 1) return;  // k_mag_ic
-  const int nh = blockIdx.x * blockDim.x + threadIdx.x;
-  double ss = 0.0, ssic = 0.0;
-  if (nh < a.H) {
-    const int l = a.hl[nh], N = a.N, L = a.L;
-    const ColView v = col_view<KL>(a, job, nh, l);
-    const size_t rst = v.rst;
-    const double2 z2 = make_double2(0.0, 0.0);
-    const double c = a.implicit;
-    // nc = c (N - N_saved) ; N_saved = N ; zerobc (tim_nlincorr, timestep.F90:696-715)
-    // vel_setbc_Tor (Re part; velocity.F90:291-299): only no-slip walls (i_vel_bc <= 2)
-    const bool tor10 = job == J_VTOR && l == 1 && a.hm[nh] == 0 && a.vel_bc <= 2;
-    const double wr = tor10 ? a.rot[ROT_OMEGA] * a.rtor10[0] : 0.0;
-    // the right-hand side in W1 (the forward pass then overwrites it row by row, in place)
-    diff_terms(v.Nn, v.S, v.W1, rst, N, c);
-    auto inC = [&](int n) {
-      if (n == 0) return tor10 ? make_double2(wr - v.X[0].x, 0.0) : z2;
-      if (n == N - 1) return z2;
-      return v.W1[(size_t)n * rst];
-    };
-    // x += d ; dterr sum of d^2 (tim_addcorr, timestep.F90:717-737)
-    auto addcorr = [&](int n, double2 d) {
-      const double2 x = v.X[(size_t)n * rst];
-      v.X[(size_t)n * rst] = make_double2(x.x + d.x, x.y + d.y);
+// The l = 0 columns of the fields that are not solved there (tim_invX skips them): N with its boundary
+// rows (predictor), x += c (N - N_saved) (corrector), by the warp of (degrees 0..31, m = 0) along n.
+// Harmonic 0 of arrays given at this lane's harmonic nh.
+template <bool CORR, class TERM>
+__device__ __forceinline__ double l0_column(int N, size_t rst, int nh, double ci, double2* X, double2* S, TERM&& term) {
+  double ss = 0.0;
+  for (int n = threadIdx.x & 31; n < N; n += 32) {
+    const ptrdiff_t id = (ptrdiff_t)(n * rst) - nh;
+    const bool wall = n == 0 || n == N - 1;
+    const double2 x = term(id), p = S[id];
+    S[id] = x;
+    if (!CORR) {
+      X[id] = wall ? make_double2(0.0, 0.0) : x;
+    } else if (!wall) {
+      const double2 o = X[id], d = make_double2(ci * (x.x - p.x), ci * (x.y - p.y));
+      X[id] = make_double2(o.x + d.x, o.y + d.y);
       ss = ss + d.x * d.x + d.y * d.y;
-    };
-    auto w1 = [&](int cc, double2 x) { v.W1[(size_t)cc * rst] = x; };
-    auto r1 = [&](int n) { return v.W1[(size_t)n * rst]; };
-    const bool zero = (job == J_COD || job == J_COMP);
-    double2 x0 = z2;
-    if (job == J_VPOL) {
-      if (l == 0) {
-        for (int n = 0; n < N; ++n) addcorr(n, inC(n));
-      } else {
-        stream_forward<KL>(v.B2, N, inC, w1);
-        stream_backward<KL>(v.B2, N, r1, [&](int cc, double2 x) { v.W2[(size_t)cc * rst] = x; });
-        auto inD = [&](int n) { return (n == 0 || n == N - 1) ? z2 : v.W2[(size_t)n * rst]; };
-        double2 xN = z2;
-        stream_forward<KL>(v.B1, N, inD, w1);
-        stream_backward<KL>(v.B1, N, r1, [&](int cc, double2 x) {
-          v.W2[(size_t)cc * rst] = x;
-          if (cc == N - 1) xN = x;
-          if (cc == 0) x0 = x;
-        });
-        double2 ca, cb;
-        gre_coeffs(v.iG, x0, xN, ca, cb);
-#pragma unroll 8
-        for (int n = 0; n < N; ++n) {
-          const double g1 = __ldg(v.g + (size_t)(2 * n) * L), g2 = __ldg(v.g + (size_t)(2 * n + 1) * L);
-          const double2 x = v.W2[(size_t)n * rst];
-          addcorr(n, make_double2(x.x - ca.x * g1 - cb.x * g2, x.y - ca.y * g1 - cb.y * g2));
-        }
-      }
-    } else if (l != 0 || zero) {
-      stream_forward<KL>(v.B1, N, inC, w1);
-      stream_backward<KL>(v.B1, N, r1, [&](int cc, double2 x) { addcorr(cc, x); if (cc == 0) x0 = x; });
-    } else {
-      for (int n = 0; n < N; ++n) addcorr(n, inC(n));
     }
-    if ((job == J_MTOR || job == J_MPOL) && l != 0) ssic = x0.x * x0.x + x0.y * x0.y;  // inner-core copy (Ni = 1)
   }
-  int slot = job == J_VTOR ? 0 : job == J_VPOL ? 1 : job == J_COD ? 2 : job == J_COMP ? 3 : job == J_MTOR ? 4 : 6;
-  warp_partial(ss, a, slot);
-  if (job == J_MTOR || job == J_MPOL) warp_partial(ssic, a, slot + 1);
+  __syncwarp();
+  return ss;
 }
 
-// The field with a conducting inner core (mag_predictor / mag_corrector, magnetic.F90:370-461;
-// tim_icinvX, timestep.F90:594-634).  Each column is one system of NL = Nic + N - 1 unknowns:
-// index c < Nic - 1 is the inner core's row c, c >= Nic - 1 the outer core's row c - (Nic - 1)
-// (c = Nic - 1, the inner-core boundary, belongs to both).  The inner core's nonlinear term
-// -rot_omega d/dphi of its field (nonlinear.F90:451-472) is formed here from the field and
-// the rate of the evaluation.  The forward pass keeps its rows in the field's two work
-// column sets (2 N >= NL rows).  grid (ceil(H / SOLVE_THREADS), 2): job row 0 toroidal,
-// 1 poloidal.  CORR: the corrector (nc = c (N - N_saved), x += correction, dterr sums).
-template <int KL, bool CORR>
-__global__ void __launch_bounds__(SOLVE_THREADS) k_mag_ic(StepArgs a) {
-  const int k = blockIdx.y, job = k == 0 ? J_MTOR : J_MPOL;
-  const int nh = blockIdx.x * blockDim.x + threadIdx.x;
-  double ss = 0.0, ssic = 0.0;
-  if (nh < a.H) {
-    const int l = a.hl[nh], N = a.N, L = a.L, Ni = a.Nic, NL = N + Ni - 1;
-    const ColView v = col_view<KL>(a, job, nh, l);
-    const size_t rst = v.rst;
-    const double2 z2 = make_double2(0.0, 0.0);
+// All fields' predictor solves (velocity.F90:369-395, codensity.F90:224-234, magnetic.F90:370-408)
+// or corrector solves (velocity.F90:413-439, codensity.F90:240-259, magnetic.F90:414-461).
+// grid ((blocks of 32 degrees) x (groups of orders), J_NJOB).
+//   X := Y X + N ; zerobc (+ setbc) ; invX          nc = c (N - N_saved) ; zerobc ; invX ; x += nc
+// The poloidal velocity solves twice: NPol through XGre, then (predictor: YPol vel_Pol +) the result
+// through XPol, then vel_gre_adjust.  Corrector partial sums, slots 0 vTor, 1 vPol, 2 cod, 3 comp,
+// 4 bTor, 5 bicTor, 6 bPol, 7 bicPol: squares of the corrections, per harmonic in the order the
+// last pass produces them, over the lanes of a warp by a fixed tree; a CTA without work writes zeros.
+//
+// IC: with a conducting inner core the field's columns (mag_predictor / mag_corrector,
+// magnetic.F90:370-461; tim_icinvX, timestep.F90:594-634) are systems of NL = Nic + N - 1 unknowns:
+// row c < Nic - 1 is the inner core's row c, c >= Nic - 1 the outer core's row c - (Nic - 1) (c = Nic - 1,
+// the inner-core boundary, belongs to both).  The inner core's nonlinear term -rot_omega d/dphi
+// of its field (nonlinear.F90:451-472) is formed from the field and the rate of the
+// evaluation.  The work rows are the outer core's in W1, the inner core's in W2 (2 N >= NL rows).
+template <int KL, bool CORR, bool IC>
+__global__ void __launch_bounds__(SOLVE_THREADS, 2) k_step_solves(StepArgs a) {
+  extern __shared__ __align__(16) unsigned char sv_sm[];
+  const int job = blockIdx.y, N = a.N;
+  const ColId c = col_id(a.L, a.M, a.Mp, a.mstart, a.bin2c);
+  const bool field = job == J_MTOR || job == J_MPOL;
+  if ((job == J_COMP && !a.comp) || cta_empty(c, a.M, a.Mp)) {
+    if (CORR) {
+      warp_partial(0.0, a, job_slot(job), c.warp);
+      if (field) warp_partial(0.0, a, job_slot(job) + 1, c.warp);
+    }
+    return;
+  }
+  const ColView v = col_view(a, job, c);
+  const size_t rst = a.H;
+  const bool zero = job == J_COD || job == J_COMP, coupled = IC && field;
+  const int q = job == J_MPOL ? 1 : 0, Ni = a.Nic;
+  cplx *icX = nullptr, *icS = nullptr;
+  SvCta k;
+  k.sm = sv_sm; k.T = blockDim.x; k.tid = threadIdx.x; k.on = c.on; k.rst = rst; k.scale = a.implicit; k.om = 0.0;
+  SvSums s{};
+  if (coupled) {
     const size_t Fi = (size_t)Ni * a.H;
-    cplx* icX = a.icstate + (size_t)k * Fi + nh;
-    cplx* icS = a.icsv + (size_t)k * Fi + nh;
-    const double om = a.rot[ROT_OMEGA_EVAL], m_ = (double)a.hm[nh], c = a.implicit;
-    auto icN = [&](int n) {  // -omega (var_coll_dph of the field)
-      const double2 x = icX[(size_t)n * rst];
-      const double dre = -(x.y * m_), dim = x.x * m_;
-      return make_double2(-om * dre, -om * dim);
-    };
-    // work rows: the outer core's in W1 (row n at cc = n + Nic - 1), the inner core's in W2
-    auto wk = [&](int cc) { return cc >= Ni - 1 ? v.W1 + (size_t)(cc - (Ni - 1)) * rst : v.W2 + (size_t)cc * rst; };
-    if (!CORR) {
-      if (l == 0) {  // not solved: the right-hand sides with their boundary rows
-        for (int n = 0; n < Ni; ++n) {
-          const double2 x = icN(n);
-          icS[(size_t)n * rst] = x;
-          icX[(size_t)n * rst] = (n == 0 || n == Ni - 1) ? z2 : x;
-        }
-        for (int n = 0; n < N; ++n) {
-          const double2 x = __ldg(v.Nn + (size_t)n * rst);
-          v.S[(size_t)n * rst] = x;
-          v.X[(size_t)n * rst] = (n == 0 || n == N - 1) ? z2 : x;
-        }
+    icX = a.icstate + (size_t)q * Fi + c.nh;
+    icS = a.icsv + (size_t)q * Fi + c.nh;
+    k.om = a.rot[ROT_OMEGA_EVAL] * (double)(c.mi * a.Mp);
+  }
+  // boundary rows of the right-hand side (tim_zerobc; cod_setbc / comp_setbc for l = 0)
+  double b0 = 0.0, bN = 0.0;
+  if (!CORR && zero && c.on && c.nh == 0) {
+    const int bc = job == J_COD ? a.cod_bc : a.comp_bc;
+    const double qi = job == J_COD ? a.qi : a.qi_comp, qo = job == J_COD ? a.qo : a.qo_comp;
+    if (bc == 1 || bc == 2) b0 = 1.0;
+    else if (bc == 3 || bc == 4) b0 = qi;
+    bN = (bc == 2 || bc == 4) ? qo : 0.0;
+  }
+  // vel_setbc_Tor (velocity.F90:291-300): the no-slip inner wall (i_vel_bc <= 2) turns with the inner core
+  if (job == J_VTOR && c.on && c.l == 1 && c.mi == 0 && a.vel_bc <= 2)
+    b0 = a.rot[ROT_OMEGA] * a.rtor10[0] - (CORR ? v.X[0].x : 0.0);
+  if (c.lb == 0 && c.mi == 0 && !zero) {
+    s.ss = l0_column<CORR>(N, rst, c.nh, a.implicit, v.X, v.S, [&](ptrdiff_t id) { return v.Nn[id]; });
+    if (coupled)  // m = 0: the inner core's term is -omega 0
+      s.ssic = l0_column<CORR>(Ni, rst, c.nh, a.implicit, icX, icS, [&](ptrdiff_t id) {
+        const double2 x = icX[id];
+        return make_double2(k.om * x.y, -(k.om * x.x));
+      });
+    if (c.l == 0) k.on = false;
+  }
+  const int fam = job_family(job);
+  const bool vpol = job == J_VPOL;
+  const double* L1 = a.lf + sv_row0(fam, c.lb, a.nlb, a.NL, KL, KL + 1);
+  const double* U1 = a.uf + sv_row0(fam, c.lb, a.nlb, a.NL, KL, 2 * KL + 2);
+  const double* L0 = a.lf + sv_row0(OP_NFAM, c.lb, a.nlb, a.NL, KL, KL + 1);
+  const ptrdiff_t up = IC ? -(ptrdiff_t)((Ni - 1) * rst) : 0;  // outer-core arrays as rows of the coupled system
+  double2 xb = make_double2(0.0, 0.0);  // the boundary point's inner-core copies
+  if (coupled && CORR && k.on) {
+    xb = icX[(size_t)(Ni - 1) * rst];
+    icS[(size_t)(Ni - 1) * rst] = make_double2(k.om * xb.y, -(k.om * xb.x));
+  }
+  const int np = vpol ? 5 : coupled && !CORR ? 4 : 2;
+  for (int i = 0; i < np; ++i) {
+    SvPass p{};
+    p.N = N;
+    p.brk = IC ? 1 << 30 : 0;
+    if (vpol) {
+      const double* L2 = a.lf + sv_row0(OP_VGRE, c.lb, a.nlb, a.NL, KL, KL + 1);
+      const double* U2 = a.uf + sv_row0(OP_VGRE, c.lb, a.nlb, a.NL, KL, 2 * KL + 2);
+      p.kind = i == 4 ? SV_GREEN : i & 1 ? SV_BWD : i == 2 && !CORR ? SV_FWDY : SV_FWD;
+      p.F = i == 0 ? L2 : i == 1 ? U2 : i == 2 ? L1 : i == 3 ? U1 : a.gf + ((size_t)c.lb * sv_rows(N, KL)) * 64;
+      p.Y = a.yf + sv_row0(fam, c.lb, a.nlb, N, KL, 2 * KL + 1);
+      p.in0 = i == 0 ? v.Nn : i & 1 ? v.W1 : i == 2 && !CORR ? v.X : v.W2;
+      p.in1 = i == 0 ? v.S : i == 2 ? v.W2 : v.X;
+      p.out = i == 4 ? v.X : i & 1 ? v.W2 : v.W1;
+      p.save = i == 0 ? v.S : nullptr;
+      p.diff = CORR && i == 0;
+      p.add = CORR && i == 4;
+      if (i == 4 && k.on) gre_coeffs(a.invg, c.l, s.x0, s.xN, p.ca, p.cb);
+    } else if (IC && coupled) {
+      if (!CORR && i < 2) {  // Y B + N of the inner (into W2), then the outer core (into W1); no elimination
+        p.kind = SV_FWDY;
+        p.F = L0;
+        p.N = i == 0 ? Ni : N;
+        p.Y = i == 0 ? a.icyf + sv_row0(q, c.lb, a.nlb, Ni, KL, 2 * KL + 1)
+                     : a.yf + sv_row0(fam, c.lb, a.nlb, N, KL, 2 * KL + 1);
+        p.in0 = i == 0 ? icX : v.X;
+        p.in1 = i == 0 ? nullptr : v.Nn;
+        p.save = i == 0 ? icS : v.S;
+        p.out = i == 0 ? v.W2 : v.W1;
+        p.rot = i == 0;
       } else {
-        // B := Y B + N (both meshes) ; zerobc ; invX
-        for (int n = 0; n < Ni; ++n) icS[(size_t)n * rst] = icN(n);
-        save_terms(v.Nn, v.S, rst, N);
-        multy_rows<KL>(v.y1, L, v.X, v.Nn, v.W1, rst, N);           // outer core: Y B + N
-        multy_rows<KL>(a.icyt + (size_t)k * Ni * (2 * KL + 1) * L + l, L, icX, icS, v.W2, rst, Ni);  // inner
-        auto in = [&](int cc) {
-          if (cc < Ni - 1) return cc == 0 ? z2 : *wk(cc);
-          const int n = cc - (Ni - 1);
-          return (n == 0 || n == N - 1) ? z2 : *wk(cc);
-        };
-        stream_forward<KL>(v.B1, NL, in, [&](int cc, double2 x) { *wk(cc) = x; });
-        stream_backward<KL>(v.B1, NL, [&](int cc) { return *wk(cc); }, [&](int cc, double2 x) {
-          if (cc <= Ni - 1) icX[(size_t)cc * rst] = x;
-          if (cc >= Ni - 1) v.X[(size_t)(cc - (Ni - 1)) * rst] = x;
-        });
+        const bool fwd = CORR ? i == 0 : i == 2;
+        p.kind = fwd ? SV_FWD : SV_BWD;
+        p.F = fwd ? L1 : U1;
+        p.N = a.NL;
+        p.brk = Ni - 1;
+        p.in0 = CORR && fwd ? icX : v.W2;
+        p.in0b = (CORR && fwd ? v.Nn : v.W1) + up;
+        p.in1 = fwd ? icS : icX;
+        p.in1b = (fwd ? v.S : v.X) + up;
+        p.save = CORR && fwd ? icS : nullptr;
+        p.saveb = CORR && fwd ? v.S + up : nullptr;
+        p.out = fwd ? v.W2 : icX;
+        p.outb = (fwd ? v.W1 : v.X) + up;
+        p.diff = CORR && fwd;
+        p.add = CORR && !fwd;
+        p.rot = CORR && fwd;
+        p.xb = xb;
       }
     } else {
-      // the right-hand side c (N - N_saved) of all NL rows in the work rows (the forward
-      // pass overwrites it in place); the saves N_saved := N of both cores
-      for (int n = 0; n < Ni; ++n) {
-        const double2 nn = icN(n), p = icS[(size_t)n * rst];
-        icS[(size_t)n * rst] = nn;
-        if (n < Ni - 1) *wk(n) = make_double2(c * (nn.x - p.x), c * (nn.y - p.y));
-      }
-      diff_terms(v.Nn, v.S, v.W1, rst, N, c);
-      auto in = [&](int cc) {
-        if (cc < Ni - 1) return cc == 0 ? z2 : *wk(cc);
-        const int n = cc - (Ni - 1);
-        return (n == 0 || n == N - 1) ? z2 : *wk(cc);
-      };
-      auto add = [&](cplx* X, double2 d) {
-        const double2 x = *X;
-        *X = make_double2(x.x + d.x, x.y + d.y);
-      };
-      if (l == 0) {
-        for (int cc = 0; cc < NL; ++cc) {
-          const double2 d = in(cc);
-          if (cc <= Ni - 1) { add(icX + (size_t)cc * rst, d); ssic = ssic + d.x * d.x + d.y * d.y; }
-          if (cc >= Ni - 1) { add(v.X + (size_t)(cc - (Ni - 1)) * rst, d); ss = ss + d.x * d.x + d.y * d.y; }
-        }
-      } else {
-        stream_forward<KL>(v.B1, NL, in, [&](int cc, double2 x) { *wk(cc) = x; });
-        stream_backward<KL>(v.B1, NL, [&](int cc) { return *wk(cc); }, [&](int cc, double2 d) {
-          if (cc <= Ni - 1) { add(icX + (size_t)cc * rst, d); ssic = ssic + d.x * d.x + d.y * d.y; }
-          if (cc >= Ni - 1) { add(v.X + (size_t)(cc - (Ni - 1)) * rst, d); ss = ss + d.x * d.x + d.y * d.y; }
-        });
-      }
+      p.kind = i == 1 ? SV_BWD : CORR ? SV_FWD : SV_FWDY;
+      p.F = i == 0 ? L1 : U1;
+      p.Y = a.yf + sv_row0(fam, c.lb, a.nlb, N, KL, 2 * KL + 1);
+      p.in0 = i == 1 ? v.W1 : CORR ? v.Nn : v.X;
+      p.in1 = i == 1 ? v.X : CORR ? v.S : v.Nn;
+      p.save = i == 0 ? v.S : nullptr;
+      p.out = i == 0 ? v.W1 : v.X;
+      p.diff = CORR && i == 0;
+      p.add = CORR && i == 1;
     }
+    p.b0 = b0;
+    p.bN = bN;
+    sv_run<KL, !CORR, true, IC>(k, p, s);
   }
-  if (CORR) {  // red slots 4 bTor, 5 bicTor, 6 bPol, 7 bicPol
-    warp_partial(ss, a, k == 0 ? 4 : 6);
-    warp_partial(ssic, a, k == 0 ? 5 : 7);
+  if (CORR) {
+    warp_partial(s.ss, a, job_slot(job), c.warp);
+    if (field) {  // Ni = 1: the inner core's copy of the boundary point
+      if (!coupled && k.on) s.ssic = s.x0.x * s.x0.x + s.x0.y * s.x0.y;
+      warp_partial(s.ssic, a, job_slot(job) + 1, c.warp);
+    }
   }
 }
 
@@ -772,43 +521,39 @@ __global__ void k_rot(double* rot, int np, int corr, double inertia, double impl
 }
 
 // Green's functions and influence matrices of the poloidal velocity (velocity.F90:148-168)
-// with the streamed solves on the solve-layout factors: thread l carries both unit
-// right-hand sides (g1 in .x: 1 at r_i; g2 in .y: 1 at r_o) through XGre, zeroes the
-// boundary rows (tim_zerobc) and solves with XPol; the passes work in place on scr [N][L].
+// with the streamed solves: lane l carries both unit right-hand sides (g1 in .x: 1 at r_i; g2
+// in .y: 1 at r_o; scr [N][Lp]) through XGre, zeroes the boundary rows (tim_zerobc)
+// and solves with XPol; the passes work in place.  One warp per block of 32 degrees.
 template <int KL>
-__global__ void k_greens(int N, int NL, int L, const double* lus, const int* ipivs, double2* scr, double* gre,
-                         double* gret, double* invg, int* fail) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l < 1 || l >= L) return;
-  constexpr int LD = 3 * KL + 1;
-  Band bg, bp;
-  bg.f = lus + (size_t)OP_VGRE * NL * LD * L + l; bg.piv = ipivs + (size_t)OP_VGRE * NL * L + l;
-  bp.f = lus + (size_t)OP_VPOL * NL * LD * L + l; bp.piv = ipivs + (size_t)OP_VPOL * NL * L + l;
-  bg.L = bp.L = L; bg.LD = bp.LD = LD;
+__global__ void __launch_bounds__(32) k_greens(int N, int NL, int L, int nlb, const double* lf, const double* uf,
+                                               double2* scr, double* gf, double* invg, int* fail) {
+  extern __shared__ __align__(16) unsigned char sv_sm[];
+  const int lb = blockIdx.x, l = lb * 32 + threadIdx.x;
+  SvCta k;
+  k.sm = sv_sm; k.T = 32; k.tid = threadIdx.x; k.on = l >= 1 && l < L; k.rst = 32 * nlb; k.scale = 1.0; k.om = 0.0;
+  SvSums s{};
   double2* w = scr + l;
-  const size_t rst = L;
-  auto unit = [&](int n) { return make_double2(n == 0 ? 1.0 : 0.0, n == N - 1 ? 1.0 : 0.0); };
-  auto rd = [&](int n) { return w[(size_t)n * rst]; };
-  auto wr = [&](int n, double2 x) { w[(size_t)n * rst] = x; };
-  stream_forward<KL>(bg, N, unit, wr);
-  stream_backward<KL>(bg, N, rd, wr);
-  w[0] = make_double2(0.0, 0.0);
-  w[(size_t)(N - 1) * rst] = make_double2(0.0, 0.0);
-  stream_forward<KL>(bp, N, rd, wr);
-  stream_backward<KL>(bp, N, rd, wr);
-  const double2 x0 = w[0], xN = w[(size_t)(N - 1) * rst];
-  double a4[4] = {x0.x, xN.x, x0.y, xN.y};  // invG(i,j) at a4[(i-1)+2(j-1)]
-  if (dev_mat_invert(2, a4, 2) != 0) atomicExch(fail, 4);
-  for (int k = 0; k < 4; ++k) invg[(size_t)l * 4 + k] = a4[k];
-  double* g1 = gre + (size_t)l * 2 * N;
-  double* g2 = g1 + N;
-  for (int n = 0; n < N; ++n) {
-    const double2 g = w[(size_t)n * rst];
-    g1[n] = g.x;
-    g2[n] = g.y;
-    gret[((size_t)n * 2 + 0) * L + l] = g.x;  // [n][2][L] copy for coalesced use in the solves
-    gret[((size_t)n * 2 + 1) * L + l] = g.y;
+  for (int i = 0; i < 4; ++i) {
+    SvPass p{};
+    p.kind = i & 1 ? SV_BWD : SV_FWD;
+    p.N = N;
+    const int fam = i < 2 ? OP_VGRE : OP_VPOL;
+    p.F = i & 1 ? uf + sv_row0(fam, lb, nlb, NL, KL, 2 * KL + 2) : lf + sv_row0(fam, lb, nlb, NL, KL, KL + 1);
+    p.in0 = w;
+    p.out = w;
+    p.unit = i == 0;
+    sv_run<KL, false, false, false>(k, p, s);
   }
+  if (!k.on) return;
+  for (int n = 0; n < N; ++n) {
+    const double2 g = w[(size_t)n * k.rst];
+    double* o = gf + ((size_t)lb * sv_rows(N, KL) + n) * 64 + threadIdx.x;
+    o[0] = g.x;
+    o[32] = g.y;
+  }
+  double a4[4] = {s.x0.x, s.xN.x, s.x0.y, s.xN.y};  // invG(i,j) at a4[(i-1)+2(j-1)]
+  if (dev_mat_invert(2, a4, 2) != 0) atomicExch(fail, 4);
+  for (int i = 0; i < 4; ++i) invg[(size_t)l * 4 + i] = a4[i];
 }
 
 // ---- energies: per-(field, category, n) sums of w_lm |a|^2 ----------------------------
@@ -897,20 +642,18 @@ SpecArgs spec_args(lsd_ctx* ctx) {
 
 StepArgs step_args(lsd_ctx* ctx) {
   StepArgs a;
-  a.N = ctx->N; a.H = ctx->H; a.KL = ctx->KL; a.L = ctx->L;
-  a.hl = ctx->d_l; a.hm = ctx->d_m;
-  a.lus = ctx->d_lus; a.ipivs = ctx->d_ipivs; a.yt = ctx->d_yt;
-  a.gret = ctx->d_gret; a.invg = ctx->d_invg;
+  a.N = ctx->N; a.H = ctx->H; a.L = ctx->L; a.nlb = ctx->nlb; a.M = ctx->M; a.Mp = ctx->Mp;
+  a.mstart = ctx->d_mstart; a.bin2c = ctx->d_bin2c;
+  a.lf = ctx->d_lf; a.uf = ctx->d_uf; a.yf = ctx->d_yf; a.gf = ctx->d_gf; a.invg = ctx->d_invg;
   a.state = ctx->d_state; a.nl = ctx->d_nl; a.sv = ctx->d_sv;
   a.work = ctx->d_spec;
   a.implicit = ctx->cfg.implicit;
   a.cod_bc = ctx->cfg.cod_bc; a.comp_bc = ctx->cfg.comp_bc; a.vel_bc = ctx->cfg.vel_bc;
   a.qi = ctx->cfg.qi; a.qo = ctx->cfg.qo; a.qi_comp = ctx->cfg.qi_comp; a.qo_comp = ctx->cfg.qo_comp;
   a.comp = ctx->cfg.comp_tstep;
-  a.red = ctx->d_red;
-  a.cpart = ctx->d_cpart; a.nwarp = (ctx->H + 31) / 32;
+  a.cpart = ctx->d_cpart; a.nwarp = ctx->nlb * ctx->M;
   a.NL = ctx->NL; a.Nic = ctx->Nic;
-  a.icstate = ctx->d_icstate; a.icsv = ctx->d_icsv; a.icyt = ctx->d_icyt;
+  a.icstate = ctx->d_icstate; a.icsv = ctx->d_icsv; a.icyf = ctx->d_icyf;
   a.rot = ctx->d_rot;
   a.rtor10 = ctx->d_r + (size_t)(3 + (ctx->nh_l1m0 >= 0 && ctx->nh_l1m0 <= 3 ? ctx->nh_l1m0 : 1)) * ctx->N;
   return a;
@@ -1062,20 +805,19 @@ int lsd_eval_marked(lsd_ctx* ctx, cudaEvent_t* marks) {
 
 namespace {
 // threads per CTA: ctx->solve_threads (a multiple of 32, at most SOLVE_THREADS; the
-// autotuner's choice); one thread per harmonic whatever the CTA size, so the results and
-// the per-warp corrector partials do not depend on it
+// autotuner's choice); one thread per harmonic and a partial-sum slot per warp of harmonics
+// whatever the CTA size, so the results do not depend on it
 template <int KL>
-void launch_pred(lsd_ctx* ctx, const StepArgs& a, bool corr) {
+int launch_solves(lsd_ctx* ctx, const StepArgs& a, bool corr) {
   const int T = ctx->solve_threads;
-  dim3 g(ceil_div(ctx->H, T), J_NJOB);
-  if (corr) k_corrector<KL><<<g, T, 0, ctx->stream>>>(a);
-  else k_predictor<KL><<<g, T, 0, ctx->stream>>>(a);
-  if (ctx->Nic > 1) {  // the field coupled to the inner core
-    dim3 gi(ceil_div(ctx->H, T), 2);
-    if (corr) k_mag_ic<KL, true><<<gi, T, 0, ctx->stream>>>(a);
-    else k_mag_ic<KL, false><<<gi, T, 0, ctx->stream>>>(a);
-    ctx->launches++;
-  }
+  const dim3 g(ctx->nlb * ceil_div(32 * ctx->M, T), J_NJOB);
+  const size_t smem = sv_smem<KL>(T);
+  const bool ic = ctx->Nic > 1;
+  auto kern = corr ? (ic ? k_step_solves<KL, true, true> : k_step_solves<KL, true, false>)
+                   : (ic ? k_step_solves<KL, false, true> : k_step_solves<KL, false, false>);
+  CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<g, T, smem, ctx->stream>>>(a);
+  return LSD_OK;
 }
 
 // rot_predictor / rot_corrector before the solves (main.F90:136, 148)
@@ -1091,14 +833,13 @@ void launch_rot(lsd_ctx* ctx, bool corr) {
 
 int launch_step_kernel(lsd_ctx* ctx, const StepArgs& a, bool corr) {
   switch (ctx->KL) {
-    case 2: launch_pred<2>(ctx, a, corr); break;
-    case 3: launch_pred<3>(ctx, a, corr); break;
-    case 4: launch_pred<4>(ctx, a, corr); break;
-    case 5: launch_pred<5>(ctx, a, corr); break;
-    case 6: launch_pred<6>(ctx, a, corr); break;
+    case 2: return launch_solves<2>(ctx, a, corr);
+    case 3: return launch_solves<3>(ctx, a, corr);
+    case 4: return launch_solves<4>(ctx, a, corr);
+    case 5: return launch_solves<5>(ctx, a, corr);
+    case 6: return launch_solves<6>(ctx, a, corr);
     default: return lsd_fail(ctx, LSD_EARG, "stencil half-width KL must be 2..6 for the step kernels");
   }
-  return LSD_OK;
 }
 }  // namespace
 
@@ -1115,7 +856,6 @@ int lsd_pred(lsd_ctx* ctx) {
 
 int lsd_corr(lsd_ctx* ctx) {
   StepArgs a = step_args(ctx);
-  cudaMemsetAsync(ctx->d_cpart, 0, sizeof(double) * 8 * a.nwarp, ctx->stream);  // slots no job writes
   launch_rot(ctx, true);
   int rc = launch_step_kernel(ctx, a, true);
   if (rc) return rc;
@@ -1742,22 +1482,27 @@ __global__ void k_state_to_coll(int N, int H, const cplx* __restrict__ in, doubl
 }
 }  // namespace
 
-int lsd_launch_greens(lsd_ctx* ctx, int* d_fail) {
-  const int N = ctx->N, NL = ctx->NL, L = ctx->L;
-  const int g = ceil_div(L, 32);
-  double2* scr = ctx->d_grescr;
-  cudaStream_t s = ctx->stream;
-  switch (ctx->KL) {
-    case 2: k_greens<2><<<g, 32, 0, s>>>(N, NL, L, ctx->d_lus, ctx->d_ipivs, scr, ctx->d_gre, ctx->d_gret, ctx->d_invg, d_fail); break;
-    case 3: k_greens<3><<<g, 32, 0, s>>>(N, NL, L, ctx->d_lus, ctx->d_ipivs, scr, ctx->d_gre, ctx->d_gret, ctx->d_invg, d_fail); break;
-    case 4: k_greens<4><<<g, 32, 0, s>>>(N, NL, L, ctx->d_lus, ctx->d_ipivs, scr, ctx->d_gre, ctx->d_gret, ctx->d_invg, d_fail); break;
-    case 5: k_greens<5><<<g, 32, 0, s>>>(N, NL, L, ctx->d_lus, ctx->d_ipivs, scr, ctx->d_gre, ctx->d_gret, ctx->d_invg, d_fail); break;
-    case 6: k_greens<6><<<g, 32, 0, s>>>(N, NL, L, ctx->d_lus, ctx->d_ipivs, scr, ctx->d_gre, ctx->d_gret, ctx->d_invg, d_fail); break;
-    default: return lsd_fail(ctx, LSD_EARG, "stencil half-width KL must be 2..6 for the step kernels");
-  }
+namespace {
+template <int KL>
+int launch_greens(lsd_ctx* ctx, int* d_fail) {
+  CUDA_TRY(cudaFuncSetAttribute(k_greens<KL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sv_smem<KL>(32)));
+  k_greens<KL><<<ctx->nlb, 32, sv_smem<KL>(32), ctx->stream>>>(ctx->N, ctx->NL, ctx->L, ctx->nlb, ctx->d_lf, ctx->d_uf,
+                                                             ctx->d_grescr, ctx->d_gf, ctx->d_invg, d_fail);
   ctx->launches++;
   CUDA_TRY(cudaGetLastError());
   return LSD_OK;
+}
+}  // namespace
+
+int lsd_launch_greens(lsd_ctx* ctx, int* d_fail) {
+  switch (ctx->KL) {
+    case 2: return launch_greens<2>(ctx, d_fail);
+    case 3: return launch_greens<3>(ctx, d_fail);
+    case 4: return launch_greens<4>(ctx, d_fail);
+    case 5: return launch_greens<5>(ctx, d_fail);
+    case 6: return launch_greens<6>(ctx, d_fail);
+    default: return lsd_fail(ctx, LSD_EARG, "stencil half-width KL must be 2..6 for the step kernels");
+  }
 }
 
 int lsd_coll_to_state(lsd_ctx* ctx, const double* re, const double* im, cplx* out) {
@@ -1790,83 +1535,72 @@ int lsd_state_to_coll_n(lsd_ctx* ctx, int rows, const cplx* in, double* re, doub
 // reference's fourth-order composite (velocity.F90:369-395, 445-465 without the Y
 // multiply): x = XPol^-1 zerobc(XGre^-1 zerobc(b)), then vel_gre_adjust with the two
 // Green's functions so that dx/dr vanishes at both walls.  In place on [N][H] complex
-// fields; one thread per harmonic and field, the rows streamed through registers.
+// fields; one thread per harmonic and field, the rows streamed (lsd_stream.cuh).
 constexpr int OPS_MAXF = 8;
 struct OpSolveArgs {
-  int N, H, L, NL;
-  const int* hl;
-  const double* lus;
-  const int* ipivs;
-  const double* gret;
+  int N, H, L, nlb, NL, M, Mp;
+  const int* mstart;
+  const int* bin2c;
+  const double *lf, *uf, *gf;
   const double* invg;
   cplx* data;  // nfield consecutive [N][H] fields
   int field[OPS_MAXF];
 };
 
 template <int KL>
-__global__ void __launch_bounds__(SOLVE_THREADS) k_opsolve(OpSolveArgs a) {
-  const int j = blockIdx.y, fld = a.field[j];
-  const int nh = blockIdx.x * blockDim.x + threadIdx.x;
-  if (nh >= a.H) return;
-  const int N = a.N, L = a.L, l = a.hl[nh];
-  constexpr int LD = 3 * KL + 1;
-  const size_t rst = a.H;
-  double2* X = a.data + (size_t)j * N * a.H + nh;
-  const double2 z2 = make_double2(0.0, 0.0);
+__global__ void __launch_bounds__(SOLVE_THREADS, 2) k_opsolve(OpSolveArgs a) {
+  extern __shared__ __align__(16) unsigned char sv_sm[];
+  const int j = blockIdx.y, fld = a.field[j], N = a.N;
+  const ColId c = col_id(a.L, a.M, a.Mp, a.mstart, a.bin2c);
+  if (cta_empty(c, a.M, a.Mp)) return;
+  SvCta k;
+  k.sm = sv_sm; k.T = blockDim.x; k.tid = threadIdx.x; k.on = c.on; k.rst = a.H; k.scale = 1.0; k.om = 0.0;
+  SvSums s{};
+  double2* X = a.data + (size_t)j * N * a.H + c.nh;
   const bool zero = fld == LSD_COD_C || fld == LSD_COMP_C;
   const int fam = fld == LSD_VEL_TOR ? OP_VTOR : fld == LSD_VEL_POL ? OP_VPOL : fld == LSD_COD_C ? OP_COD
                 : fld == LSD_COMP_C ? OP_COMP : fld == LSD_MAG_TOR ? OP_MTOR : OP_MPOL;
-  auto band = [&](int f) {
-    Band B;
-    B.f = a.lus + (size_t)f * a.NL * LD * L + l;
-    B.piv = a.ipivs + (size_t)f * a.NL * L + l;
-    B.L = L;
-    B.LD = LD;
-    return B;
-  };
-  auto in = [&](int n) { return (n == 0 || n == N - 1) ? z2 : X[(size_t)n * rst]; };  // tim_zerobc
-  auto rd = [&](int n) { return X[(size_t)n * rst]; };
-  auto wr = [&](int c, double2 x) { X[(size_t)c * rst] = x; };
-  if (l == 0 && !zero) {
-    X[0] = z2;
-    X[(size_t)(N - 1) * rst] = z2;
-    return;
+  if (k.on && c.l == 0 && !zero) {
+    X[0] = X[(size_t)(N - 1) * k.rst] = make_double2(0.0, 0.0);
+    k.on = false;
   }
-  const Band B1 = band(fam);
-  if (fld == LSD_VEL_POL) {
-    const Band B2 = band(OP_VGRE);
-    stream_forward<KL>(B2, N, in, wr);
-    stream_backward<KL>(B2, N, rd, wr);
-    double2 x0 = z2, xN = z2;
-    stream_forward<KL>(B1, N, in, wr);
-    stream_backward<KL>(B1, N, rd, [&](int c, double2 x) {
-      X[(size_t)c * rst] = x;
-      if (c == N - 1) xN = x;
-      if (c == 0) x0 = x;
-    });
-    double iG[4];
-    for (int i = 0; i < 4; ++i) iG[i] = __ldg(a.invg + (size_t)l * 4 + i);
-    double2 ca, cb;
-    gre_coeffs(iG, x0, xN, ca, cb);
-    const double* g = a.gret + l;
-#pragma unroll 8
-    for (int n = 0; n < N; ++n) {
-      const double g1 = __ldg(g + (size_t)(2 * n) * L), g2 = __ldg(g + (size_t)(2 * n + 1) * L);
-      const double2 x = X[(size_t)n * rst];
-      X[(size_t)n * rst] = make_double2(x.x - ca.x * g1 - cb.x * g2, x.y - ca.y * g1 - cb.y * g2);
-    }
-    return;
+  const bool vpol = fld == LSD_VEL_POL;
+  const int np = vpol ? 5 : 2;
+  for (int i = 0; i < np; ++i) {  // in place: forward, backward (poloidal velocity: XGre, XPol, Green's functions)
+    SvPass p{};
+    const int f = vpol && i < 2 ? OP_VGRE : fam;
+    p.kind = i == 4 ? SV_GREEN : i & 1 ? SV_BWD : SV_FWD;
+    p.N = N;
+    p.F = i == 4 ? a.gf + (size_t)c.lb * sv_rows(N, KL) * 64
+        : i & 1 ? a.uf + sv_row0(f, c.lb, a.nlb, a.NL, KL, 2 * KL + 2)
+                : a.lf + sv_row0(f, c.lb, a.nlb, a.NL, KL, KL + 1);
+    p.in0 = X;
+    p.out = X;
+    if (i == 4 && k.on) gre_coeffs(a.invg, c.l, s.x0, s.xN, p.ca, p.cb);
+    sv_run<KL, false, true, false>(k, p, s);
   }
-  stream_forward<KL>(B1, N, in, wr);
-  stream_backward<KL>(B1, N, rd, wr);
 }
+
+namespace {
+template <int KL>
+int launch_opsolve(lsd_ctx* ctx, const OpSolveArgs& a, int nfield) {
+  const int T = ctx->solve_threads;
+  const size_t smem = sv_smem<KL>(T);
+  CUDA_TRY(cudaFuncSetAttribute(k_opsolve<KL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k_opsolve<KL><<<dim3(ctx->nlb * ceil_div(32 * ctx->M, T), nfield), T, smem, ctx->stream>>>(a);
+  ctx->launches++;
+  CUDA_TRY(cudaGetLastError());
+  return LSD_OK;
+}
+}  // namespace
 
 int lsd_operator_solve(lsd_ctx* ctx, int nfield, const int* fields, double* d_data) {
   if (nfield < 1 || nfield > OPS_MAXF) return lsd_fail(ctx, LSD_EARG, "lsd_operator_solve_device: 1..8 fields");
   if (!ctx->have_ops) return lsd_fail(ctx, LSD_ESTATE, "lsd_operator_solve_device: no operators built");
   OpSolveArgs a;
-  a.N = ctx->N; a.H = ctx->H; a.L = ctx->L; a.NL = ctx->NL;
-  a.hl = ctx->d_l; a.lus = ctx->d_lus; a.ipivs = ctx->d_ipivs; a.gret = ctx->d_gret; a.invg = ctx->d_invg;
+  a.N = ctx->N; a.H = ctx->H; a.L = ctx->L; a.nlb = ctx->nlb; a.NL = ctx->NL; a.M = ctx->M; a.Mp = ctx->Mp;
+  a.mstart = ctx->d_mstart; a.bin2c = ctx->d_bin2c;
+  a.lf = ctx->d_lf; a.uf = ctx->d_uf; a.gf = ctx->d_gf; a.invg = ctx->d_invg;
   a.data = (cplx*)d_data;
   for (int i = 0; i < OPS_MAXF; ++i) a.field[i] = LSD_COD_C;
   for (int i = 0; i < nfield; ++i) {
@@ -1877,19 +1611,14 @@ int lsd_operator_solve(lsd_ctx* ctx, int nfield, const int* fields, double* d_da
       return lsd_fail(ctx, LSD_EARG, "lsd_operator_solve_device: the field's operators are coupled to the inner core (Nic > 1)");
     a.field[i] = f;
   }
-  const int T = ctx->solve_threads;
-  const dim3 g(ceil_div(ctx->H, T), nfield);
   switch (ctx->KL) {
-    case 2: k_opsolve<2><<<g, T, 0, ctx->stream>>>(a); break;
-    case 3: k_opsolve<3><<<g, T, 0, ctx->stream>>>(a); break;
-    case 4: k_opsolve<4><<<g, T, 0, ctx->stream>>>(a); break;
-    case 5: k_opsolve<5><<<g, T, 0, ctx->stream>>>(a); break;
-    case 6: k_opsolve<6><<<g, T, 0, ctx->stream>>>(a); break;
+    case 2: return launch_opsolve<2>(ctx, a, nfield);
+    case 3: return launch_opsolve<3>(ctx, a, nfield);
+    case 4: return launch_opsolve<4>(ctx, a, nfield);
+    case 5: return launch_opsolve<5>(ctx, a, nfield);
+    case 6: return launch_opsolve<6>(ctx, a, nfield);
     default: return lsd_fail(ctx, LSD_EARG, "stencil half-width KL must be 2..6");
   }
-  ctx->launches++;
-  CUDA_TRY(cudaGetLastError());
-  return LSD_OK;
 }
 
 int lsd_factor_batch(lsd_ctx* ctx, int n, int kl, int nmat, double* d_ab, int* d_ipiv, int* d_info) {

@@ -10,6 +10,7 @@
 
 #include "lsd_banded.cuh"
 #include "lsd_common.cuh"
+#include "lsd_stream.cuh"
 
 namespace {
 
@@ -447,25 +448,31 @@ __global__ void k_build_ops(int N, int NL, int KL, int L, int wpb, const double*
 #undef MB
 }
 
-// LAPACK layouts [fam][L][N][band] -> solve layouts [fam][N][band][L] (degree fastest),
-// for the factors, the pivots and the Y bands
-// (factors and pivots with the row stride NL; the field families of a conducting inner
-// core have NL rows, the others N)
-__global__ void k_lu_transpose(int N, int NL, int icfam, int KL, int L, const double* lu, const int* ipiv,
-                               const double* y, double* lus, int* ipivs, double* yt) {
-  int l = blockIdx.x * blockDim.x + threadIdx.x;
-  int j = blockIdx.y;
-  int fam = blockIdx.z;
+// LAPACK layouts [fam][L][N][band] -> the solve layouts of lsd_stream.cuh, for the factors (with
+// the reciprocals of U's diagonal), the pivots' offsets and the Y bands by rows (factors and
+// pivots with NL rows a family; the field families of a conducting inner core have NL rows, the
+// others N).  One thread per (degree, row, family).
+__global__ void k_solve_layouts(int N, int NL, int icfam, int KL, int L, int nlb, const double* lu, const int* ipiv,
+                                const double* y, double* lf, double* uf, double* yf) {
+  const int l = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, fam = blockIdx.z;
   if (l >= L) return;
   const bool coupled = icfam && (fam == OP_MTOR || fam == OP_MPOL);
   if (j >= (coupled ? NL : N)) return;
-  const int ld = 3 * KL + 1, ldm = 2 * KL + 1;
+  const int ld = 3 * KL + 1, ldm = 2 * KL + 1, lb = l >> 5, lane = l & 31;
   const double* A = lu + (((size_t)fam * L + l) * NL + j) * ld;
-  for (int row = 0; row < ld; ++row) lus[(((size_t)fam * NL + j) * ld + row) * L + l] = A[row];
-  ipivs[((size_t)fam * NL + j) * L + l] = ipiv[((size_t)fam * L + l) * NL + j];
+  double* F = lf + sv_row0(fam, lb, nlb, NL, KL, KL + 1) + (size_t)j * (KL + 1) * 32 + lane;
+  for (int i = 0; i < KL; ++i) F[i * 32] = A[ldm + i];
+  F[KL * 32] = __longlong_as_double((long long)(ipiv[((size_t)fam * L + l) * NL + j] - 1 - j));
+  double* U = uf + sv_row0(fam, lb, nlb, NL, KL, 2 * KL + 2) + (size_t)j * (2 * KL + 2) * 32 + lane;
+  for (int i = 0; i <= 2 * KL; ++i) U[i * 32] = A[2 * KL - i];
+  U[(2 * KL + 1) * 32] = 1.0 / A[2 * KL];
   if (j >= N) return;
-  const double* Y = y + (((size_t)fam * L + l) * N + j) * ldm;
-  for (int row = 0; row < ldm; ++row) yt[(((size_t)fam * N + j) * ldm + row) * L + l] = Y[row];
+  const double* Y = y + ((size_t)fam * L + l) * N * ldm;
+  double* W = yf + sv_row0(fam, lb, nlb, N, KL, ldm) + (size_t)j * ldm * 32 + lane;
+  for (int t = 0; t < ldm; ++t) {
+    const int jj = j - KL + t;
+    W[t * 32] = jj >= 0 && jj < N ? Y[(size_t)jj * ldm + (ldm - 1 - t)] : 0.0;
+  }
 }
 
 // The field's operators with a conducting inner core, Boussinesq (tim_iclumesh_Tor_X /
@@ -473,11 +480,11 @@ __global__ void k_lu_transpose(int N, int NL, int icfam, int KL, int L, const do
 // N - 1 unknowns, 1..Ni on the inner core's mesh and Ni..NL on the outer core's (Ni the
 // inner-core boundary, shared); row 1 the innermost point's condition, row Ni the
 // continuity of dr across the boundary, row NL the insulating exterior.  Also the inner
-// core's Y bands (tim_mesh_Y on its mesh) in the solve layout [k][Ni][2KL+1][L].
+// core's Y bands (tim_mesh_Y on its mesh) as Y rows of the solve layout.
 // One warp per (l, k), k = 0 toroidal, 1 poloidal, in shared memory as k_build_ops.
-__global__ void k_build_icops(int N, int Ni, int KL, int L, int wpb, const double* r, const double* dr,
+__global__ void k_build_icops(int N, int Ni, int KL, int L, int nlb, int wpb, const double* r, const double* dr,
                               const double* radlap, const double* icr, const double* icdr, const double* icradlap,
-                              OpParams P, const double* dtp, double* lu, int* ipiv, double* icyt, int* info) {
+                              OpParams P, const double* dtp, double* lu, int* ipiv, double* icyf, int* info) {
   extern __shared__ double osm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int l = blockIdx.x * wpb + warp, k = blockIdx.y;
@@ -551,7 +558,9 @@ __global__ void k_build_icops(int N, int Ni, int KL, int L, int wpb, const doubl
         const double t = ll1 * icrm2[j - 1];
         v = v + c1_ - c2y * (t + P.Hyp * t * t);
       }
-      icyt[(((size_t)k * Ni + (j - 1)) * ldm + (row - 1)) * L + l] = v;
+      const int n = j - 1 + row - 1 - KL;  // v is the entry of row n on X(j - 1)
+      if (n >= 0 && n < Ni)
+        icyf[sv_row0(k, l >> 5, nlb, Ni, KL, ldm) + ((size_t)n * ldm + (ldm - row)) * 32 + (l & 31)] = v;
     }
   (void)icband;
 #undef AX
@@ -684,14 +693,13 @@ int lsd_launch_operator_build(lsd_ctx* ctx, const double* dtp, int* status) {
   if (Ni > 1) {  // the field families coupled to the inner core
     CUDA_TRY(cudaFuncSetAttribute(k_build_icops, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemi));
     k_build_icops<<<dim3(ceil_div(L, wpbi), 2), 32 * wpbi, smemi, s>>>(
-        N, Ni, KL, L, wpbi, ctx->d_r, ctx->d_dr, ctx->d_radlap, ctx->d_icr, ctx->d_icdr, ctx->d_icradlap, P, dtp,
-        ctx->d_lu, ctx->d_ipiv, ctx->d_icyt, ctx->d_info);
+        N, Ni, KL, L, ctx->nlb, wpbi, ctx->d_r, ctx->d_dr, ctx->d_radlap, ctx->d_icr, ctx->d_icdr, ctx->d_icradlap, P, dtp,
+        ctx->d_lu, ctx->d_ipiv, ctx->d_icyf, ctx->d_info);
     ctx->launches++;
   }
   dim3 gt(ceil_div(L, 64), NL, OP_NFAM);
-  k_lu_transpose<<<gt, 64, 0, s>>>(N, NL, Ni > 1 ? 1 : 0, KL, L, ctx->d_lu, ctx->d_ipiv, ctx->d_y, ctx->d_lus,
-                                   ctx->d_ipivs, ctx->d_yt);
-  CUDA_TRY(cudaMemsetAsync(ctx->d_gret, 0, sizeof(double) * 2 * N * L, s));
+  k_solve_layouts<<<gt, 64, 0, s>>>(N, NL, Ni > 1 ? 1 : 0, KL, L, ctx->nlb, ctx->d_lu, ctx->d_ipiv, ctx->d_y, ctx->d_lf,
+                                    ctx->d_uf, ctx->d_yf);
   {
     int rc = lsd_launch_greens(ctx, ctx->d_opfail);  // on the solve-layout factors
     if (rc) return rc;
