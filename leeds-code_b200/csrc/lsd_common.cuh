@@ -250,7 +250,7 @@ void lsd_ozaki_get_tiles(const lsd_ctx* ctx, int* nst, int* ctas);
 int lsd_ozaki_set_tiles(lsd_ctx* ctx, int nst, int ctas);
 // ---- autotuner (lsd_tune.cu) ----
 bool lsd_fft_compiled(int E, int G);
-size_t lsd_products_smem_for(int nfields, int P2, int E, int G, int NM);
+size_t lsd_products_smem_for(int nfields, int E, int G);
 int lsd_autotune(lsd_ctx* ctx);
 
 // small helpers

@@ -288,11 +288,15 @@ __device__ __forceinline__ void col_pass(double2* rows, int nrows, const FFTTabs
   }
 }
 
-// Row pass: a G-point DFT over the G contiguous values of each (row, t1).  In place.
-template <int E, int G, int SIGN, int RS = E * (G + 1)>
+// Row pass: a G-point DFT over the G contiguous values of each (row, t1).  In place.  Neighbouring
+// lanes take neighbouring t1 (stride G + 1, odd for G > 1), or with ROWS neighbouring rows (an odd RS;
+// ROWS: the rows padded to lanes): distinct banks either way, but t1 runs out after E lanes and
+// the next row's offset then collides.
+template <int E, int G, int SIGN, int RS = E * (G + 1), int ROWS = 0>
 __device__ __forceinline__ void row_pass(double2* rows, int nrows, const FFTTabs& t) {
-  for (int i = threadIdx.x; i < nrows * E; i += blockDim.x) {
-    const int r = i / E, t1 = i - r * E;
+  for (int i = threadIdx.x; i < (ROWS ? ROWS : nrows) * E; i += blockDim.x) {
+    const int r = ROWS ? i % (ROWS ? ROWS : 1) : i / E, t1 = ROWS ? i / (ROWS ? ROWS : 1) : i - r * E;
+    if (ROWS && r >= nrows) continue;
     double2* seg = rows + (size_t)r * RS + t1 * (G + 1);
     double2 v[G];
 #pragma unroll
@@ -465,25 +469,79 @@ __device__ __forceinline__ void prod_point(const double* v, double* o, const Pro
   }
 }
 
-// grid (2 HB, N): one half-row h = blockIdx.x (its southern and northern theta row) per
-// CTA, 256 threads, up to two CTAs per SM so that one's memory waits overlap the other's
-// work.  The inputs are gathered bin by bin (bin -> m-counter map, L1-cached) straight into
-// the packed half spectra of the padded rows [NF][2][E (G+1)] (NF = inputs + derived rows),
-// so the load phase has no barrier; barriers separate only the FFT passes and products.
-constexpr int PROD_THREADS = 256;
+// One half-row h = blockIdx.x (its southern and northern theta row) of shell blockIdx.y per CTA, up
+// to two CTAs per SM so that one's memory waits overlap the other's work.
+//
+// The E and O rows of a field are transformed as they are: the transform is linear, so the
+// southern and northern samples are e + o and e - o at the products, and the results' folded
+// sums go into the forward transform.  The column passes take a pair of columns (k1, G - k1) per
+// thread (k1 = 0 and G/2, their own partners, together): the pair holds every bin k with its
+// mirror P2 - k, so the half-spectrum packing (and, behind the forward transform, the
+// unpacking) happens in registers between global memory and the E-point DFTs.  Bins >= M = 2 P2 / 3
+// are zero: 2 E / 3 rows of a column are loaded, all of a thread's loads in flight at once, before
+// the tables are ready.  What bounds it: the shared-memory passes (per input row one write, one read
+// and write, one read; packing and unpacking through shared memory took three more) and the
+// latency of the gather.
+// At lmax 127, Nr 129 (1.12 GB in and out) 0.75 ms; with packing and unpacking as shared-memory passes of
+// their own 0.83.  Anelastic with composition at L = 96 0.60 ms for both sets (0.72).
+// Rows [2 NF][RSP], RSP odd so that the column pass's lanes (one row each) write distinct banks.
+__host__ __device__ constexpr int prod_rsp(int E, int G) { return (E * (G + 1)) | 1; }
+__host__ __device__ constexpr int prod_lanes(int rows) { return rows < 8 ? rows : (rows + 7) / 8 * 8; }
+__host__ __device__ constexpr size_t prod_tab_bytes(int E, int G) { return sizeof(double2) * (2 * (size_t)E * G + E + G); }
+__host__ __device__ constexpr size_t prod_smem(int nf, int E, int G) {
+  return sizeof(double2) * 2 * (size_t)nf * prod_rsp(E, G) + prod_tab_bytes(E, G);
+}
+template <int E, int G, int PS> struct ProdCfg {
+  static constexpr int NF = PSet<PS>::in + PSet<PS>::deriv, NPAIR = G > 1 ? G / 2 : 1;
+  // lanes run over the rows, padded to a multiple of 8 (the lanes of one 128-byte access) where
+  // there are that many, so that an access never mixes two columns, whose banks would collide
+  static constexpr int RIN = prod_lanes(2 * NF), ROUT = prod_lanes(2 * PSet<PS>::out);
+  static constexpr int ITEMS = RIN * NPAIR;
+  // one column pair per thread where that is up to 384 threads
+  static constexpr int THREADS = ITEMS <= 256 || ITEMS > 384 ? 256 : ITEMS;
+  // two CTAs per SM where the rows fit twice and the two columns' registers (96 up to E = 6, else 120;
+  // 128 at E = 12) do too: at E = 9 with 320 threads the spills of a second CTA cost 6 %
+  static constexpr int MINB = E <= 12 && prod_smem(NF, E, G) <= 112 * 1024 && THREADS * (E <= 6 ? 96 : 120) <= 32768 ? 2 : 1;
+};
+
+// m-counter of FFT bin m (the folded order: counters 2 j and 2 j + 1 are the orders j and M - 1 - j)
+__device__ __forceinline__ int bin_counter(int m, int M) { return m < M / 2 ? 2 * m : 2 * (M - 1 - m) + 1; }
+
+// Z[k] and Z[P2-k] of the c2r packing from Y[k], Y[P2-k]; w = e^{2 pi i k / Ph} (w^(P2-k) = -conj w)
+__device__ __forceinline__ void pack_pair(double2 yk, double2 ym, double2 w, double2& zk, double2& zm) {
+  const double2 yc = conj2(ym), s = add2(yk, yc), wd = cmul(w, sub2(yk, yc));
+  zk = make_double2(s.x - wd.y, s.y + wd.x);
+  zm = make_double2(s.x + wd.y, wd.x - s.y);
+}
+// X[k] and X[P2-k] of the r2c unpacking from Z[k], Z[P2-k]
+__device__ __forceinline__ void unpack_pair(double2 zk, double2 zm, double2 w, double2& xk, double2& xm) {
+  const double2 zc = conj2(zm);
+  const double2 A = make_double2(0.5 * (zk.x + zc.x), 0.5 * (zk.y + zc.y));
+  const double2 Bi = make_double2(0.5 * (zk.x - zc.x), 0.5 * (zk.y - zc.y));
+  const double2 B = cmulc(make_double2(Bi.y, -Bi.x), w);
+  xk = add2(A, B);
+  xm = conj2(sub2(A, B));
+}
 
 template <int E, int G, int PS>
-__global__ void __launch_bounds__(PROD_THREADS, 2) k_products(FFTPlanDev pl, int N, ProdConst pc,
-                                                              const cplx* four_in, cplx* four_out) {
-  constexpr int RS = E * (G + 1), P2 = E * G;
-  constexpr int NF_IN = PSet<PS>::in, NDER = PSet<PS>::deriv, NF = NF_IN + NDER, NF_OUT = PSet<PS>::out;
+__global__ void __launch_bounds__(ProdCfg<E, G, PS>::THREADS, ProdCfg<E, G, PS>::MINB)
+    k_products(FFTPlanDev pl, int N, ProdConst pc, const cplx* four_in, cplx* four_out) {
+  constexpr int RSP = prod_rsp(E, G), P2 = E * G, K2 = 2 * E / 3;
+  constexpr int NF_IN = PSet<PS>::in, NF = ProdCfg<E, G, PS>::NF, NF_OUT = PSet<PS>::out;
+  constexpr int NPAIR = ProdCfg<E, G, PS>::NPAIR, ITEMS = ProdCfg<E, G, PS>::ITEMS, NT = ProdCfg<E, G, PS>::THREADS;
+  constexpr int RIN = ProdCfg<E, G, PS>::RIN, ROUT = ProdCfg<E, G, PS>::ROUT;
   extern __shared__ __align__(16) unsigned char psm[];
   const int n = blockIdx.y, h = blockIdx.x, hb = h >> 1, jj = h & 1;
   const int NM = pl.NM, M = pl.M, Th = pl.Th, Th2 = pl.Th2;
   if (h >= Th2) return;  // padding half-row of an odd Th2
-  double2* rows = (double2*)psm;                 // [NF][2][RS]
-  const FFTTabs tabs = fft_tabs_init<E, G>((unsigned char*)(rows + (size_t)NF * 2 * RS), pl);
-  const int BLK = NM * 4;                        // one field's (n, h/2) block
+  double2* rows = (double2*)psm;  // [NF][E/O][RSP]
+  FFTTabs tabs;
+  tabs.tw = rows + 2 * NF * RSP;
+  tabs.twE = tabs.tw + P2;
+  tabs.twG = tabs.twE + E;
+  tabs.twh = tabs.twG + G;
+  tabs.thm = tabs.b2c = nullptr;
+  const int BLK = NM * 4;  // one field's (n, h/2) block
   const size_t fstride = (size_t)N * pl.HB * BLK;
   const size_t boff = ((size_t)n * pl.HB + hb) * BLK + jj;  // element (c, p) at boff + 2 (2c + p)
   const int tid = threadIdx.x;
@@ -496,86 +554,97 @@ __global__ void __launch_bounds__(PROD_THREADS, 2) k_products(FFTPlanDev pl, int
     sh.rm1 = pc.r[(size_t)2 * N + n]; sh.rinv = sh.rm1; sh.rrr = pc.r[(size_t)4 * N + n];
     sh.Cmag = pc.Pm / (pc.E * sh.rho);
   }
-  // ---- gather + pack, no barrier: item (f, k), k = 0 .. P2/2, loads the (E, O) pairs of
-  // bins k and P2-k (counters bin2c[.]) once, straight from this half-row's block, forms the
-  // southern (E + O) and northern (E - O) half spectra and writes the packed rows at
-  // positions k and P2-k (k = 0: position 0, whose partner is the Nyquist bin P2 >= M;
-  // k = P2/2: its own partner).  Bins >= M are zero (dealiasing).  Batches of U items per
-  // thread keep their loads in flight.
-  constexpr int KH = P2 / 2 + 1, U = 3, NITEM = NF_IN * KH;
-  auto put = [&](int row, int k, double2 yk, double2 ym) {
-    rows[(size_t)row * RS + ppos<G>(k)] = c2r_pack(k, yk, ym, tabs.twh);
-    if (k != 0 && 2 * k != P2) rows[(size_t)row * RS + ppos<G>(P2 - k)] = c2r_pack(P2 - k, ym, yk, tabs.twh);
+  // ---- gather: item (column pair q, row 2 f + p); pair 0 are columns 0 and G/2
+  double2 A[K2], B[K2];
+  auto gather = [&](int it) {
+    const int q = it / RIN, row = it - q * RIN, f = row >> 1, p = row & 1;
+    const int a = q, b = q ? G - q : G / 2;
+    if (f >= NF) return;
+    if (f < NF_IN) {
+      const cplx* src = four_in + (size_t)pc.fin[f] * fstride + boff + 2 * p;
+#pragma unroll
+      for (int i = 0; i < K2; ++i) {
+        A[i] = src[4 * bin_counter(a + G * i, M)];
+        if (G > 1) B[i] = src[4 * bin_counter(b + G * i, M)];
+      }
+    } else if constexpr (PSet<PS>::deriv > 0) {
+      // qv1, qv2 from the u_th (input 1), u_ph (input 2) bins: cot theta is odd about the
+      // equator and swaps E and O, 1/sin theta keeps them
+      const double s1 = pc.sn1[h], cot = pc.gp[h] * s1;
+      const bool first = f == NF_IN;
+      const cplx* keep = four_in + (size_t)pc.fin[first ? 2 : 1] * fstride + boff + 2 * p;
+      const cplx* swap = four_in + (size_t)pc.fin[first ? 1 : 2] * fstride + boff + 2 * (1 - p);
+      const double cs = first ? cot : -cot;
+      auto val = [&](int m) {
+        const int c = 4 * bin_counter(m, M);
+        const double2 x = keep[c], y = swap[c];
+        const double mk = (double)(m * pl.Mp) * s1;  // i mk x + cs y
+        return make_double2(sh.rinv * (cs * y.x - mk * x.y), sh.rinv * (cs * y.y + mk * x.x));
+      };
+#pragma unroll
+      for (int i = 0; i < K2; ++i) {
+        A[i] = val(a + G * i);
+        if (G > 1) B[i] = val(b + G * i);
+      }
+    }
   };
-  for (int it0 = tid; it0 < NITEM; it0 += U * PROD_THREADS) {
-    double2 e0[U], o0[U], e1[U], o1[U];
+  // ---- pack and the E-point DFTs of both columns (inverse column pass)
+  auto columns = [&](int it) {
+    const int q = it / RIN, row = it - q * RIN;
+    const int a = q, b = q ? G - q : G / 2;
+    if (row >= 2 * NF) return;
+    const double2 z0 = make_double2(0.0, 0.0);
+    double2 Za[E], Zb[E];
+    if (q) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int it = it0 + u * PROD_THREADS;
-      e0[u] = o0[u] = e1[u] = o1[u] = make_double2(0.0, 0.0);
-      if (it < NITEM) {
-        const int f = it / KH, k = it - f * KH, km = k == 0 ? P2 : P2 - k;
-        const cplx* src = four_in + (size_t)pc.fin[f] * fstride + boff;
-        if (k < M) {
-          const int c = tabs.b2c[k];
-          e0[u] = src[4 * c]; o0[u] = src[4 * c + 2];
-        }
-        if (km < M) {
-          const int c = tabs.b2c[km];
-          e1[u] = src[4 * c]; o1[u] = src[4 * c + 2];
-        }
+      for (int i = 0; i < E; ++i)
+        pack_pair(i < K2 ? A[i < K2 ? i : 0] : z0, E - 1 - i < K2 ? B[E - 1 - i < K2 ? E - 1 - i : 0] : z0,
+                  tabs.twh[a + G * i], Za[i], Zb[E - 1 - i]);
+    } else {  // the imaginary part of bin 0 is ignored, its mirror is the Nyquist bin (0)
+      double2 x;
+      Za[0] = make_double2(A[0].x, A[0].x);
+#pragma unroll
+      for (int i = 1; i <= (E - 1) / 2; ++i)
+        pack_pair(A[i], E - i < K2 ? A[E - i < K2 ? E - i : 0] : z0, tabs.twh[G * i], Za[i], Za[E - i]);
+      if (E % 2 == 0) pack_pair(A[E / 2], A[E / 2], tabs.twh[P2 / 2], Za[E / 2], x);
+      if (G > 1) {
+#pragma unroll
+        for (int i = 0; i < E / 2; ++i)
+          pack_pair(B[i], E - 1 - i < K2 ? B[E - 1 - i < K2 ? E - 1 - i : 0] : z0, tabs.twh[G / 2 + G * i], Zb[i],
+                    Zb[E - 1 - i]);
+        if (E % 2 == 1) pack_pair(B[E / 2], B[E / 2], tabs.twh[P2 / 2], Zb[E / 2], x);
       }
     }
+    double2* out = rows + row * RSP;
+    rdft<E, E, +1>(Za, tabs.twE);
+    out[a] = Za[0];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int it = it0 + u * PROD_THREADS;
-      if (it < NITEM) {
-        const int f = it / KH, k = it - f * KH;
-        put(f * 2, k, add2(e0[u], o0[u]), add2(e1[u], o1[u]));
-        put(f * 2 + 1, k, sub2(e0[u], o0[u]), sub2(e1[u], o1[u]));
-      }
+    for (int t = 1; t < E; ++t) out[t * (G + 1) + a] = cmul(Za[t], tabs.tw[t * G + a]);
+    if (G > 1) {
+      rdft<E, E, +1>(Zb, tabs.twE);
+      out[b] = Zb[0];
+#pragma unroll
+      for (int t = 1; t < E; ++t) out[t * (G + 1) + b] = cmul(Zb[t], tabs.tw[t * G + b]);
     }
+  };
+  if (tid < ITEMS) gather(tid);
+  for (int i = tid; i < P2; i += NT) {
+    tabs.tw[i] = __ldg(&pl.tw2[(i / G) * (i % G)]);
+    tabs.twh[i] = __ldg(&pl.twh[i]);
   }
-  if constexpr (NDER > 0) {  // the qv1, qv2 rows from the u_th (input 1), u_ph (input 2) bins
-    const cplx* sth = four_in + (size_t)pc.fin[1] * fstride + boff;
-    const cplx* sph = four_in + (size_t)pc.fin[2] * fstride + boff;
-    for (int k = tid; k < KH; k += PROD_THREADS) {  // bins k and P2-k, both sides
-      const int km = k == 0 ? P2 : P2 - k;
-      double2 te[2], to[2], pe[2], po[2];
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int b = q ? km : k;
-        te[q] = to[q] = pe[q] = po[q] = make_double2(0.0, 0.0);
-        if (b < M) {
-          const int c = tabs.b2c[b];
-          te[q] = sth[4 * c]; to[q] = sth[4 * c + 2]; pe[q] = sph[4 * c]; po[q] = sph[4 * c + 2];
-        }
-      }
-#pragma unroll
-      for (int side = 0; side < 2; ++side) {
-        const int j = row_theta(h, side, Th);
-        const double s1 = pc.sn1[j], cot = pc.gp[j] * s1;
-        double2 q1[2], q2[2];
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const double2 t = side ? sub2(te[q], to[q]) : add2(te[q], to[q]);
-          const double2 p = side ? sub2(pe[q], po[q]) : add2(pe[q], po[q]);
-          const double mk = (double)((q ? km : k) * pl.Mp) * s1;
-          q1[q] = make_double2(sh.rinv * (cot * t.x - mk * p.y), sh.rinv * (cot * t.y + mk * p.x));
-          q2[q] = make_double2(sh.rinv * (-mk * t.y - cot * p.x), sh.rinv * (mk * t.x - cot * p.y));
-        }
-        put(NF_IN * 2 + side, k, q1[0], q1[1]);
-        put((NF_IN + 1) * 2 + side, k, q2[0], q2[1]);
-      }
-    }
+  for (int i = tid; i < E; i += NT) tabs.twE[i] = __ldg(&pl.tw2[G * i]);
+  for (int i = tid; i < G; i += NT) tabs.twG[i] = __ldg(&pl.tw2[E * i]);
+  __syncthreads();
+  if (tid < ITEMS) columns(tid);
+  for (int it = tid + NT; it < ITEMS; it += NT) {
+    gather(it);
+    columns(it);
   }
   __syncthreads();
-  // ---- inverse FFTs of the 2 NF rows
-  col_pass<E, G, +1>(rows, NF * 2, tabs);
+  row_pass<E, G, +1, RSP, RIN>(rows, NF * 2, tabs);
   __syncthreads();
-  row_pass<E, G, +1>(rows, NF * 2, tabs);
-  __syncthreads();
-  // ---- products at every point (row side, sample position, part re/im), in place into 0..NF_OUT-1
+  // ---- products: item (sample position, Re / Im part = one of two neighbouring samples), both rows;
+  // the folded results over the first 2 NF_OUT rows, in place
   const double scale = 1.0 / (double)pl.Ph;
   constexpr bool HAS_UB = (PS == PS_BOUSS || PS == PS_BOUSS_COMP || PS == PS_ANEL_MOM);
   double cmr = 0.0, cmh = 0.0, cdr2 = 0.0, cdh2 = 0.0, EPm = 0.0;
@@ -595,38 +664,38 @@ __global__ void __launch_bounds__(PROD_THREADS, 2) k_products(FFTPlanDev pl, int
   // once)
   double tv = 0.0, tm = 0.0;
   const bool torque = (PS == PS_BOUSS || PS == PS_BOUSS_COMP) && pc.rotsum && n == 0;
-  for (int i = tid; i < 2 * P2; i += PROD_THREADS) {
-    const int r = i / P2, pos = ppos<G>(i - r * P2);
-    const int j = row_theta(h, r, Th);
-    const double sn = pc.sn[j], cs = pc.gp[j];
-    const bool tq = torque && !(r == 1 && (Th & 1) && h == Th2 - 1);
-    double2 v[NF];
+  const bool equator = (Th & 1) && h == Th2 - 1;  // odd Th: the equator row is counted once
+  const int jn = row_theta(h, 1, Th);
+  const double sn0 = pc.sn[h], cs0 = pc.gp[h], sn1 = pc.sn[jn], cs1 = pc.gp[jn];
+  for (int i = tid; i < 2 * P2; i += NT) {
+    double* d = (double*)rows + 2 * ppos<G>(i >> 1) + (i & 1);
+    double v[2][NF], o[2][NF_OUT];
 #pragma unroll
-    for (int f = 0; f < NF; ++f) v[f] = rows[(size_t)(f * 2 + r) * RS + pos];
-    double2 out[NF_OUT];
-#pragma unroll
-    for (int part = 0; part < 2; ++part) {
-      double x[NF], o[NF_OUT];
-#pragma unroll
-      for (int f = 0; f < NF; ++f) x[f] = part == 0 ? v[f].x : v[f].y;
-      if constexpr (HAS_UB)
-        if (pc.cflmax) cfl_point(x, EPm, pc.E, pc.Pm, cdr2, cdh2, cmr, cmh);
-      if (tq) {
-        const double gw = pc.gwP0[j];
-        tv = tv + gw * ((pc.rotS * x[2] - x[4]) * sn);
-        tm = tm + gw * ((x[6] * x[8]) * sn);
-      }
-      prod_point<PS>(x, o, pc, sh, sn, cs);
-#pragma unroll
-      for (int q = 0; q < NF_OUT; ++q) {
-        if (part == 0) out[q].x = o[q] * scale; else out[q].y = o[q] * scale;
-      }
+    for (int f = 0; f < NF; ++f) {
+      const double e = d[2 * (2 * f) * RSP], q = d[2 * (2 * f + 1) * RSP];
+      v[0][f] = e + q;
+      v[1][f] = e - q;
     }
 #pragma unroll
-    for (int q = 0; q < NF_OUT; ++q) rows[(size_t)(q * 2 + r) * RS + pos] = out[q];
+    for (int r = 0; r < 2; ++r) {
+      if constexpr (HAS_UB)
+        if (pc.cflmax) cfl_point(v[r], EPm, pc.E, pc.Pm, cdr2, cdh2, cmr, cmh);
+      if (HAS_UB && torque && !(r == 1 && equator)) {
+        const double gw = pc.gwP0[r ? jn : h], sn = r ? sn1 : sn0;
+        tv = tv + gw * ((pc.rotS * v[r][2] - v[r][4]) * sn);
+        tm = tm + gw * ((v[r][6] * v[r][8]) * sn);
+      }
+      prod_point<PS>(v[r], o[r], pc, sh, r ? sn1 : sn0, r ? cs1 : cs0);
+    }
+#pragma unroll
+    for (int q = 0; q < NF_OUT; ++q) {
+      const double s0 = o[0][q] * scale, s1 = o[1][q] * scale;
+      d[2 * (2 * q) * RSP] = equator ? 0.5 * (s0 + s1) : s0 + s1;
+      d[2 * (2 * q + 1) * RSP] = s0 - s1;
+    }
   }
   if (torque) {  // this CTA's two sums, in a fixed order, into its slots of rotsum
-    __shared__ double tq[2][PROD_THREADS / 32];
+    __shared__ double tq[2][NT / 32];
     for (int o = 16; o > 0; o >>= 1) {
       tv += __shfl_down_sync(0xffffffffu, tv, o);
       tm += __shfl_down_sync(0xffffffffu, tm, o);
@@ -635,7 +704,7 @@ __global__ void __launch_bounds__(PROD_THREADS, 2) k_products(FFTPlanDev pl, int
     __syncthreads();
     if (tid < 2) {
       double t = 0.0;
-      for (int w = 0; w < PROD_THREADS / 32; ++w) t = t + tq[tid][w];
+      for (int w = 0; w < NT / 32; ++w) t = t + tq[tid][w];
       pc.rotsum[2 * h + tid] = t;
     }
   }
@@ -652,23 +721,62 @@ __global__ void __launch_bounds__(PROD_THREADS, 2) k_products(FFTPlanDev pl, int
     }
   }
   __syncthreads();
-  // ---- forward FFTs of the product rows (spectrum back in natural order)
-  row_pass<E, G, -1>(rows, NF_OUT * 2, tabs);
+  // ---- forward: row pass, then the column pairs of the result rows with the unpacking, stored to
+  // the analysis layout (neighbouring lanes hold E and O of an output: whole 32-byte sectors)
+  row_pass<E, G, -1, RSP, ROUT>(rows, NF_OUT * 2, tabs);
   __syncthreads();
-  col_pass<E, G, -1>(rows, NF_OUT * 2, tabs);
-  __syncthreads();
-  // ---- unpack bins, fold south/north into E/O, store: a thread per (output, counter)
-  // unpacks both rows once and writes the (E, O) pair, neighbours in four_off_a, with one
-  // 32-byte store (the field bases are 32-byte aligned)
-  const bool equator = (Th & 1) && h == Th2 - 1;  // odd Th: the equator row is counted once
-  for (int i = tid; i < NF_OUT * NM; i += PROD_THREADS) {
-    const int q = i / NM, c = i - q * NM;
-    const int b = tabs.thm[c];
-    const double2 xs = row_unpack<G>(rows + (size_t)(q * 2) * RS, b, P2, tabs.twh);
-    const double2 xn = row_unpack<G>(rows + (size_t)(q * 2 + 1) * RS, b, P2, tabs.twh);
-    double2 ev = add2(xs, xn);
-    if (equator) { ev.x *= 0.5; ev.y *= 0.5; }
-    st_global_2c(four_out + (size_t)q * fstride + four_off_a(n, c, 0, h, N, Th2), ev, sub2(xs, xn));
+  for (int it = tid; it < ROUT * NPAIR; it += NT) {
+    const int q = it / ROUT, row = it - q * ROUT;
+    if (row >= 2 * NF_OUT) continue;
+    const int a = q, b = q ? G - q : G / 2;
+    const double2* in = rows + row * RSP;
+    double2 Za[E], Zb[E];
+    Za[0] = in[a];
+#pragma unroll
+    for (int t = 1; t < E; ++t) Za[t] = cmulc(in[t * (G + 1) + a], tabs.tw[t * G + a]);
+    rdft<E, E, -1>(Za, tabs.twE);
+    if (G > 1) {
+      Zb[0] = in[b];
+#pragma unroll
+      for (int t = 1; t < E; ++t) Zb[t] = cmulc(in[t * (G + 1) + b], tabs.tw[t * G + b]);
+      rdft<E, E, -1>(Zb, tabs.twE);
+    }
+    cplx* out = four_out + (size_t)(row >> 1) * fstride + ((size_t)n * Th2 + h) * 2 + (row & 1);
+    const size_t cst = (size_t)N * Th2 * 2;  // four_off_a's stride of a counter
+    auto put = [&](int m, double2 x) { out[bin_counter(m, M) * cst] = x; };
+    double2 x, y;
+    if (q) {
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        unpack_pair(Za[i], Zb[E - 1 - i], tabs.twh[a + G * i], x, y);
+        if (i < K2) put(a + G * i, x);
+        if (E - 1 - i < K2) put(b + G * (E - 1 - i), y);
+      }
+    } else {
+      put(0, make_double2(Za[0].x + Za[0].y, 0.0));
+#pragma unroll
+      for (int i = 1; i <= (E - 1) / 2; ++i) {
+        unpack_pair(Za[i], Za[E - i], tabs.twh[G * i], x, y);
+        put(G * i, x);
+        if (E - i < K2) put(G * (E - i), y);
+      }
+      if (E % 2 == 0) {
+        unpack_pair(Za[E / 2], Za[E / 2], tabs.twh[P2 / 2], x, y);
+        put(P2 / 2, x);
+      }
+      if (G > 1) {
+#pragma unroll
+        for (int i = 0; i < E / 2; ++i) {
+          unpack_pair(Zb[i], Zb[E - 1 - i], tabs.twh[G / 2 + G * i], x, y);
+          put(G / 2 + G * i, x);
+          if (E - 1 - i < K2) put(G / 2 + G * (E - 1 - i), y);
+        }
+        if (E % 2 == 1) {
+          unpack_pair(Zb[E / 2], Zb[E / 2], tabs.twh[P2 / 2], x, y);
+          put(P2 / 2, x);
+        }
+      }
+    }
   }
 }
 
@@ -838,14 +946,12 @@ int dispatch_EG(int E, int G, F&& f) {
 bool lsd_fft_compiled(int E, int G) { return dispatch_EG(E, G, [](auto, auto) { return 0; }) == 0; }
 
 // shared memory of the products kernel with the plan (E, G) for nfields staged rows
-size_t lsd_products_smem_for(int nfields, int P2, int E, int G, int NM) {
-  return sizeof(double2) * ((size_t)nfields * 2 * E * (G + 1)) + fft_tab_bytes(P2, E, G, NM);
-}
+size_t lsd_products_smem_for(int nfields, int E, int G) { return prod_smem(nfields, E, G); }
 size_t lsd_products_smem_eg(const lsd_ctx* ctx, int E, int G) {
   const bool comp = ctx->cfg.comp_tstep != 0;
   int nf = comp ? 18 : 15;
   if (!ctx->cfg.boussinesq) nf = (comp ? 18 : 15) + 2;
-  return lsd_products_smem_for(nf, ctx->P2, E, G, ctx->NM);
+  return lsd_products_smem_for(nf, E, G);
 }
 
 // P2 = E G with G the power-of-two part of P2 capped at 16; (E, G) must be instantiated.
@@ -899,15 +1005,13 @@ namespace {
 template <int PS>
 int launch_products_set(lsd_ctx* ctx, const ProdConst& pc, const cplx* four_in, cplx* four_out) {
   FFTPlanDev pl = make_plan(ctx);
-  constexpr int NF = PSet<PS>::in + PSet<PS>::deriv;
-  const size_t smem = sizeof(double2) * ((size_t)NF * 2 * ctx->fftE * (ctx->fftG + 1)) +
-                      fft_tab_bytes(ctx->P2, ctx->fftE, ctx->fftG, ctx->NM);
+  const size_t smem = prod_smem(PSet<PS>::in + PSet<PS>::deriv, ctx->fftE, ctx->fftG);
   if (smem > 224 * 1024) return lsd_fail(ctx, LSD_EARG, "products: FFT rows do not fit in shared memory");
   dim3 grid(2 * ctx->HB, ctx->N);
   int rc = dispatch_EG(ctx->fftE, ctx->fftG, [&](auto e, auto g) {
     constexpr int E = decltype(e)::value, G = decltype(g)::value;
     cudaFuncSetAttribute(k_products<E, G, PS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_products<E, G, PS><<<grid, PROD_THREADS, smem, ctx->stream>>>(pl, ctx->N, pc, four_in, four_out);
+    k_products<E, G, PS><<<grid, ProdCfg<E, G, PS>::THREADS, smem, ctx->stream>>>(pl, ctx->N, pc, four_in, four_out);
     return 0;
   });
   if (rc) return lsd_fail(ctx, LSD_EARG, "FFT length not supported");

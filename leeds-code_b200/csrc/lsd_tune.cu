@@ -27,7 +27,7 @@ int products_fields(const lsd_config& c) {
 // the candidates of a configuration, the default of each list first
 void tune_space(const lsd_config& c, lsd_tune_space& sp) {
   std::memset(&sp, 0, sizeof(sp));
-  const int P2 = c.M * 3 / 2, NM = 2 * ((c.M + 1) / 2);
+  const int P2 = c.M * 3 / 2;
   int G = 1;
   while (G < 16 && P2 % (2 * G) == 0) G *= 2;
   const int nf = products_fields(c);
@@ -35,7 +35,7 @@ void tune_space(const lsd_config& c, lsd_tune_space& sp) {
     if (P2 % g) continue;
     const int E = P2 / g;
     if (!lsd_fft_compiled(E, g)) continue;
-    if (lsd_products_smem_for(nf, P2, E, g, NM) > 224 * 1024) continue;
+    if (lsd_products_smem_for(nf, E, g) > 224 * 1024) continue;
     sp.fft_E[sp.nfft] = E;
     sp.fft_G[sp.nfft] = g;
     sp.nfft++;
