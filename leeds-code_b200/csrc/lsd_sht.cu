@@ -29,8 +29,10 @@
 // copies (16-byte, 8-byte where an odd Th2 misaligns the tables), three CTAs per SM.  What bounds
 // it: the FP64 tensor pipe at large L, the ring's first fill where a counter has few K.
 // At lmax 127, Nr 129 (one evaluation: 4 vector syntheses and a gradient, 2 vector and a scalar
-// analysis) 0.53 ms at 57 % of the pipe and 0.32 ms at 76 %; thread-tiled products with a theta row
+// analysis) 0.47 ms at 60 % of the pipe and 0.30 ms at 80 %; thread-tiled products with a theta row
 // or a harmonic per thread took 3.37 and 1.40 ms (2.8 and 3.2 TF/s, waiting for their tables).
+#include <type_traits>
+
 #include "lsd_common.cuh"
 
 namespace {
@@ -59,6 +61,7 @@ struct LegClass {
 };
 struct LegArgs {
   int N, H, Th2, NM, HB, mtiles;
+  int cols[LG_MAXCLASS];  // column blocks of each class
   const int* mstart;
   const int* mlen;
   const int* hm;
@@ -68,7 +71,8 @@ struct LegArgs {
 };
 
 __device__ __forceinline__ uint32_t lg_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-// asynchronous copies of 16 / 8 bytes; valid = false writes zeros and reads nothing
+// asynchronous copies of 16 / 8 bytes; valid = false writes zeros and reads nothing (the address may
+// then lie outside the array)
 __device__ __forceinline__ void cp16(void* dst, const void* src, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(lg_smem(dst)), "l"(src), "r"(valid ? 16 : 0)
                : "memory");
@@ -84,52 +88,85 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
 }
 
 template <bool ANAL, bool VEC>
-__device__ __forceinline__ void leg_tile(const LegArgs& a, const LegClass& k, double* sm) {
+__device__ __forceinline__ void leg_tile(const LegArgs& a, const LegClass& k, int col, int cm, double* sm) {
   constexpr int NTAB = VEC ? 2 : 1, SH = VEC ? 16 : 32;  // shells of a CTA's 64 columns
   constexpr int TAB = ANAL ? LG_TAB_A : LG_TAB_S, STAGE = LG_DATA + 2 * TAB;
-  const int c = blockIdx.x / a.mtiles, m0 = (blockIdx.x - c * a.mtiles) * LG_BM;
-  const int nsh = k.ng * a.N, s0 = blockIdx.y * SH;
+  const int c = cm / a.mtiles, m0 = (cm - c * a.mtiles) * LG_BM;
+  const int nsh = k.ng * a.N, s0 = col * SH;
   const int kbeg = a.mstart[c], klen = a.mlen[c], Th2 = a.Th2;
-  if (s0 >= nsh || (ANAL && 2 * m0 >= klen)) return;
+  if (ANAL && 2 * m0 >= klen) return;
   const int tid = threadIdx.x, lane = tid & 31, par = tid >> 6, half = (tid >> 5) & 1;
   const int lk = lane & 3, lq = lane >> 2;
   // M rows of this warp: theta rows m0 .. (synthesis), harmonics par + 2 (m0 ..) (analysis)
   const int mrows = ANAL ? (klen + 1 - par) / 2 - m0 : Th2 - m0;
   const int klast = ANAL ? 2 * Th2 : klen;  // staged values per (shell, field) row
   const int nch = (klast + 15) / 16;
+  const int neg = (lq & 3) == 1 || (lq & 3) == 2 ? (int)0x80000000 : 0;  // sign of segment 2's column lq & 3
 
-  // this thread copies value e of every chunk of the staged rows r0 + 8 i
+  // Copies: addresses are formed once, a chunk only advances them (the index arithmetic of a
+  // chunk took six integer instructions per matrix instruction).  Data: value e of the staged
+  // rows r0 + 8 i.
   const int e = tid & 15;
   const cplx* src[4];
+  int live = 0;  // bit i: the row exists
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int row = (tid >> 4) + 8 * i, s = s0 + (VEC ? row >> 1 : row), f = VEC ? row & 1 : 0;
     const int g = s / a.N, n = s - g * a.N;
-    src[i] = s < nsh ? k.in[f][g] + (ANAL ? four_off_a(n, c, 0, 0, a.N, Th2) : (size_t)n * a.H + kbeg) + e : nullptr;
+    src[i] = k.in[f][s < nsh ? g : 0] + (ANAL ? four_off_a(n, c, 0, 0, a.N, Th2) : (size_t)n * a.H + kbeg) + e;
+    live |= (s < nsh ? 1 : 0) << i;
   }
+  // Tables: row tr (+ trs i), doubles tj (+ tjs i) of the tile: 16 rows (kk) x 48 theta, 8 threads a row
+  // (synthesis), 96 rows (harmonics) x 8 theta, 4 threads a row of 16-byte, 8 of 8-byte copies
   const bool even = (Th2 & 1) == 0;
+  const int tw = even ? 2 : 1, tper = ANAL ? 8 / tw : 8;  // doubles a copy, threads a row
+  const int tr = tid / tper, tj = (tid & (tper - 1)) * tw;
+  const double* tsrc = a.leg + ((size_t)k.tab[0] * a.H + kbeg + (ANAL ? 2 * m0 : 0) + tr) * Th2 + (ANAL ? 0 : m0) + tj;
+  const ptrdiff_t t2 = VEC ? (ptrdiff_t)(k.tab[1] - k.tab[0]) * a.H * Th2 : 0;  // T2 - T1
+  const int tdst = tr * (ANAL ? LG_AA : LG_AS) + tj;
   auto issue = [&](int ch) {
     if (ch < nch) {
       double* st = sm + (ch % LG_STAGES) * STAGE;
+      const bool in = ch * 16 + e < klast;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const bool ok = src[i] && ch * 16 + e < klast;
-        cp16(st + 2 * (((tid >> 4) + 8 * i) * LG_DROW + e), ok ? (const void*)(src[i] + ch * 16) : (const void*)a.leg, ok);
-      }
-      double* tb = st + LG_DATA;
-      // table rows: kk x 48 theta (synthesis), harmonic x 8 theta (analysis)
-      auto rows = [&](auto cp, int W) {
-        const int per = (ANAL ? 8 : LG_BM) / W, nrow = ANAL ? 2 * LG_BM : 16;
-        for (int i = tid; i < NTAB * nrow * per; i += LG_THREADS) {
-          const int u = i % per, r = (i / per) % nrow, t = i / (per * nrow);
-          const int kk = ANAL ? 2 * m0 + r : ch * 16 + r, j = (ANAL ? ch * 8 : m0) + W * u;
-          const bool ok = kk < klen && j < Th2;
-          const double* p = ok ? a.leg + ((size_t)k.tab[t] * a.H + kbeg + kk) * Th2 + j : a.leg;
-          cp(tb + t * TAB + r * (ANAL ? LG_AA : LG_AS) + W * u, p, ok);
+      for (int i = 0; i < 4; ++i)
+        cp16(st + 2 * (((tid >> 4) + 8 * i) * LG_DROW + e), src[i] + ch * 16, in && ((live >> i) & 1));
+      double* tb = st + LG_DATA + tdst;
+      if (ANAL) {
+        const double* p = tsrc + ch * 8;
+        const bool jin = ch * 8 + tj < Th2;
+        const int rest = klen - 2 * m0 - tr;  // rows of this counter from tr on
+        if (even) {
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int t = 0; t < NTAB; ++t)
+              cp16(tb + t * TAB + 32 * i * LG_AA, p + t * t2 + (ptrdiff_t)(32 * i) * Th2, jin && 32 * i < rest);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 6; ++i)
+#pragma unroll
+            for (int t = 0; t < NTAB; ++t)
+              cp8(tb + t * TAB + 16 * i * LG_AA, p + t * t2 + (ptrdiff_t)(16 * i) * Th2, jin && 16 * i < rest);
         }
-      };
-      if (even) rows([](double* d, const double* p, bool ok) { cp16(d, p, ok); }, 2);
-      else rows([](double* d, const double* p, bool ok) { cp8(d, p, ok); }, 1);
+      } else {
+        const double* p = tsrc + (ptrdiff_t)(ch * 16) * Th2;
+        const bool rin = ch * 16 + tr < klen;
+        const int rest = Th2 - m0 - tj;
+        if (even) {
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int t = 0; t < NTAB; ++t)
+              cp16(tb + t * TAB + 16 * i, p + t * t2 + 16 * i, rin && 16 * i < rest);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 6; ++i)
+#pragma unroll
+            for (int t = 0; t < NTAB; ++t)
+              cp8(tb + t * TAB + 8 * i, p + t * t2 + 8 * i, rin && 8 * i < rest);
+        }
+      }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -146,35 +183,40 @@ __device__ __forceinline__ void leg_tile(const LegArgs& a, const LegClass& k, do
     __syncthreads();  // chunk ch has landed for every thread; chunk ch - 1's stage is free
     issue(ch + LG_STAGES - 1);
     const double* st = sm + (ch % LG_STAGES) * STAGE;
+    auto multiply = [&](auto full) {  // full: no M tile to leave out
 #pragma unroll
-    for (int seg = 0; seg < NTAB; ++seg) {
-      const int dp = VEC && seg == 0 ? 1 - par : par;  // parity of the data of this segment
-      const double* tb = st + LG_DATA + seg * TAB;
+      for (int seg = 0; seg < NTAB; ++seg) {
+        const int dp = VEC && seg == 0 ? 1 - par : par;  // parity of the data of this segment
+        const double* tb = st + LG_DATA + seg * TAB;
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {  // four K each
-        const int ki = dp + 2 * (4 * q + lk);
-        double b[LG_NT];
+        for (int q = 0; q < 2; ++q) {  // four K of each parity
+          if (ch * 16 + 8 * q >= klast) break;
+          const int ki = dp + 2 * (4 * q + lk);
+          double b[LG_NT];
 #pragma unroll
-        for (int j = 0; j < LG_NT; ++j) {
-          const int col = half * 32 + j * 8 + lq;
-          if (VEC) {  // columns: Re, Im of out0, Re, Im of out1 of a shell
-            const int comp = col & 3, f = seg ? 1 - (comp >> 1) : comp >> 1, part = seg ? 1 - (comp & 1) : comp & 1;
-            const double x = st[2 * (((col >> 2) * 2 + f) * LG_DROW + ki) + part];
-            b[j] = seg && (comp == 1 || comp == 2) ? -x : x;
-          } else {
-            b[j] = st[2 * ((col >> 1) * LG_DROW + ki) + (col & 1)];
+          for (int j = 0; j < LG_NT; ++j) {
+            const int col = half * 32 + j * 8 + lq;
+            if (VEC) {  // columns: Re, Im of out0, Re, Im of out1 of a shell
+              const int comp = col & 3, f = seg ? 1 - (comp >> 1) : comp >> 1, part = seg ? 1 - (comp & 1) : comp & 1;
+              const double x = st[2 * (((col >> 2) * 2 + f) * LG_DROW + ki) + part];
+              b[j] = seg ? __hiloint2double(__double2hiint(x) ^ neg, __double2loint(x)) : x;
+            } else {
+              b[j] = st[2 * ((col >> 1) * LG_DROW + ki) + (col & 1)];
+            }
           }
-        }
 #pragma unroll
-        for (int i = 0; i < LG_MT; ++i) {
-          if (i * 8 < mrows) {
-            const double av = ANAL ? tb[(par + 2 * (i * 8 + lq)) * LG_AA + 4 * q + lk] : tb[ki * LG_AS + i * 8 + lq];
+          for (int i = 0; i < LG_MT; ++i) {
+            if (decltype(full)::value || i * 8 < mrows) {
+              const double av = ANAL ? tb[(par + 2 * (i * 8 + lq)) * LG_AA + 4 * q + lk] : tb[ki * LG_AS + i * 8 + lq];
 #pragma unroll
-            for (int j = 0; j < LG_NT; ++j) dmma(acc[i][j], av, b[j]);
+              for (int j = 0; j < LG_NT; ++j) dmma(acc[i][j], av, b[j]);
+            }
           }
         }
       }
-    }
+    };
+    if (mrows >= LG_BM) multiply(std::true_type());
+    else multiply(std::false_type());
   }
 
   // accumulators: M row lq, columns 2 lk, 2 lk + 1 (Re, Im) of each tile
@@ -190,26 +232,33 @@ __device__ __forceinline__ void leg_tile(const LegArgs& a, const LegClass& k, do
 #pragma unroll
       for (int i = 0; i < LG_MT; ++i)
         if (i * 8 + lq < mrows) out[2 * (m0 + i * 8 + lq)] = make_double2(acc[i][j][0], zero ? 0.0 : acc[i][j][1]);
-    } else {
+    } else {  // theta rows m0 + 8 i + lq: 4 half-row pairs of four_off apart
       const int po = k.flip ? 1 - par : par;
+      cplx* o = out + four_off(n, c, po, m0 + lq, a.NM, a.HB);
+      const size_t step = (size_t)a.NM * 16;
       const double f = k.scale ? a.rinv[n] : 1.0;
 #pragma unroll
       for (int i = 0; i < LG_MT; ++i)
         if (i * 8 + lq < mrows) {
           const double x = acc[i][j][0] * f, y = acc[i][j][1] * f;
-          out[four_off(n, c, po, m0 + i * 8 + lq, a.NM, a.HB)] = k.rot ? make_double2(-y, x) : make_double2(x, y);
+          o[i * step] = k.rot ? make_double2(-y, x) : make_double2(x, y);
         }
     }
   }
 }
 
-// grid (counters x M tiles, column blocks of the largest class, classes)
+// grid: (counters x M tiles) of every column block of every class, one class after another (a grid
+// of the largest class's column blocks for all classes spent 8 % on CTAs without work)
 template <bool ANAL>
 __global__ void __launch_bounds__(LG_THREADS, 3) k_leg(LegArgs a) {
   extern __shared__ __align__(16) double lg_sm[];
-  const LegClass& k = a.k[blockIdx.z];
-  if (k.vec) leg_tile<ANAL, true>(a, k, lg_sm);
-  else leg_tile<ANAL, false>(a, k, lg_sm);
+  const int per = a.NM * a.mtiles;
+  int col = blockIdx.x / per, z = 0;
+  const int cm = blockIdx.x - col * per;
+  while (col >= a.cols[z]) col -= a.cols[z++];
+  const LegClass& k = a.k[z];
+  if (k.vec) leg_tile<ANAL, true>(a, k, col, cm, lg_sm);
+  else leg_tile<ANAL, false>(a, k, col, cm, lg_sm);
 }
 
 // The classes of a launch: add() opens a class for its tables or joins the open one.
@@ -241,18 +290,24 @@ template <bool ANAL>
 int launch_leg(lsd_ctx* ctx, LegBuilder& b) {
   if (b.nc == 0) return LSD_OK;
   LegArgs& a = b.a;
+  for (int i = 1; i < b.nc; ++i)  // the vector class, whose tiles are the longest, first
+    if (a.k[i].vec && !a.k[0].vec) {
+      const LegClass t = a.k[0];
+      a.k[0] = a.k[i];
+      a.k[i] = t;
+    }
   a.N = ctx->N; a.H = ctx->H; a.Th2 = ctx->Th2; a.NM = ctx->NM; a.HB = ctx->HB;
   a.mstart = ctx->d_mstart; a.mlen = ctx->d_mlen; a.hm = ctx->d_m; a.leg = ctx->d_leg; a.rinv = ctx->d_rinv;
   int klmax = 0, cols = 0;
   for (int c = 0; c < ctx->NM; ++c) klmax = ctx->mlen[c] > klmax ? ctx->mlen[c] : klmax;
   a.mtiles = ANAL ? ceil_div((klmax + 1) / 2, LG_BM) : ceil_div(ctx->Th2, LG_BM);
   for (int i = 0; i < b.nc; ++i) {
-    const int n = ceil_div(a.k[i].ng * ctx->N, a.k[i].vec ? 16 : 32);
-    cols = n > cols ? n : cols;
+    a.cols[i] = ceil_div(a.k[i].ng * ctx->N, a.k[i].vec ? 16 : 32);
+    cols += a.cols[i];
   }
   const size_t smem = sizeof(double) * LG_STAGES * (LG_DATA + 2 * (ANAL ? LG_TAB_A : LG_TAB_S));
   CUDA_TRY(cudaFuncSetAttribute(k_leg<ANAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_leg<ANAL><<<dim3(ctx->NM * a.mtiles, cols, b.nc), LG_THREADS, smem, ctx->stream>>>(a);
+  k_leg<ANAL><<<ctx->NM * a.mtiles * cols, LG_THREADS, smem, ctx->stream>>>(a);
   ctx->launches++;
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return lsd_fail(ctx, LSD_ECUDA, std::string("k_leg: ") + cudaGetErrorString(e));
