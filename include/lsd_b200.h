@@ -68,8 +68,10 @@ extern "C" {
 #define LSD_LEG_GWLLSIN1MP 7
 
 /* precision of the Legendre contraction */
-#define LSD_PREC_FP64   0   /* plain FP64 on the CUDA cores                              */
-#define LSD_PREC_OZAKI  1   /* FP64 emulated by int8 slices on tcgen05 tensor cores      */
+#define LSD_PREC_FP64   0   /* FP64 products and sums (the FP64 tensor instruction)      */
+#define LSD_PREC_OZAKI  1   /* at least the precision of ozaki_slices int8 slices: the slices
+                               on the tcgen05 tensor cores (up to five), from six on FP64
+                               where that is faster (all but large analyses at six)      */
 
 /* energy diagnostics written by lsd_energies (io.F90:1739-2024 column order) */
 #define LSD_E_TIME     0   /* tim_t                                                      */

@@ -241,6 +241,8 @@ int lsd_ozaki_setup(lsd_ctx* ctx);
 void lsd_ozaki_free(lsd_ctx* ctx);
 int lsd_ozaki_check(lsd_ctx* ctx);
 int* lsd_ozaki_err_flag(lsd_ctx* ctx);
+bool lsd_ozaki_use_synth(const lsd_ctx* c);  // the int8 slices are the faster contraction here
+bool lsd_ozaki_use_anal(const lsd_ctx* c);
 int lsd_ozaki_launch_synth(lsd_ctx* ctx, const SynthGroup* groups, int ngroups);
 int lsd_ozaki_launch_anal(lsd_ctx* ctx, const AnalGroup* groups, int ngroups);
 bool lsd_ozaki_tiles_ok(int S, int nst, int ctas);

@@ -14,6 +14,7 @@
 // (row max x column max).
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "lsd_common.cuh"
@@ -836,26 +837,48 @@ constexpr int OZ_MAXG_SYNTH = OZ_MAXG, OZ_MAXG_ANAL = 4;  // groups per launch
 // the digit / exponent buffer of each type's chain
 int oz_buf(int type) { return type == OZ_VEC || type == OZ_ST ? 0 : type == OZ_P || type == OZ_Q ? 1 : 2; }
 
-// f(k_oz_gemm<TYPE, S>) for the runtime slice count S
+// f(integral_constant S) for the runtime slice count S; nothing for the counts at which the type's
+// contractions run on the FP64 instruction (lsd_ozaki_use_synth / _anal)
 template <int TYPE, class F>
-void oz_gemm_dispatch(int S, F&& f) {
+void oz_slices_dispatch(int S, F&& f) {
   switch (S) {
-    case 2: f(k_oz_gemm<TYPE, 2>); break;
-    case 3: f(k_oz_gemm<TYPE, 3>); break;
-    case 4: f(k_oz_gemm<TYPE, 4>); break;
-    case 5: f(k_oz_gemm<TYPE, 5>); break;
-    case 6: f(k_oz_gemm<TYPE, 6>); break;
-    case 7: f(k_oz_gemm<TYPE, 7>); break;
-    default: f(k_oz_gemm<TYPE, 8>); break;
+    case 2: f(std::integral_constant<int, 2>()); break;
+    case 3: f(std::integral_constant<int, 3>()); break;
+    case 4: f(std::integral_constant<int, 4>()); break;
+    case 5: f(std::integral_constant<int, 5>()); break;
+    case 6: if constexpr (OzT<TYPE>::anal) f(std::integral_constant<int, 6>()); break;
+    default: break;
   }
 }
 template <int TYPE>
 void oz_set_smem(int S, size_t smem) {
-  oz_gemm_dispatch<TYPE>(S, [&](auto kern) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  oz_slices_dispatch<TYPE>(S, [&](auto sc) {
+    cudaFuncSetAttribute(k_oz_gemm<TYPE, decltype(sc)::value>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
 }
 }  // namespace
+
+// Which contraction an LSD_PREC_OZAKI context runs: the int8 slices, or the FP64 tensor instruction
+// (lsd_sht.cu), which is exact to FP64 and costs the same for every S.  One evaluation (four vector
+// syntheses and a gradient; two vector and a scalar analysis), us, FP64 against S slices:
+//   L = M, N     FP64         S = 2       3           4           5           6           7
+//   64,  65     55 +  43     83 + 57     83 + 59     86 + 61     93 + 66    105 + 66    116 + 72
+//   96,  97    221 + 113    207 + 133   210 + 139   220 + 145   234 + 158   264 + 164   297 + 182
+//   128, 129   471 + 301    411 + 266   430 + 277   451 + 289   494 + 307   555 + 320   666 + 344
+//   192, 97   1055 + 602    935 + 494   970 + 516  1084 + 547  1153 + 602  1235 + 641  1452 + 721
+//   256, 65   1569 + 917   1448 + 596  1563 + 648  1657 + 707  1737 + 787  2029 + 871  2268 + 989
+// From six slices on the S (S + 1) / 2 digit products and the slicing pass cost more than the FP64
+// products at every size but one: six slices in the analysis above L = 192, whose slicing pass over
+// the theta rows is spread over the most harmonics.  Up to five slices the int8 path stays at all
+// sizes: a caller who asked for 38 bits gets the rounding of 38 bits.
+bool lsd_ozaki_use_synth(const lsd_ctx* c) {
+  const OzState* o = (const OzState*)c->oz;
+  return o && o->S <= 5;
+}
+bool lsd_ozaki_use_anal(const lsd_ctx* c) {
+  const OzState* o = (const OzState*)c->oz;
+  return o && (o->S <= 5 || (o->S == 6 && c->L > 192));
+}
 
 void lsd_ozaki_free(lsd_ctx* ctx) {
   OzState* o = (OzState*)ctx->oz;
@@ -969,6 +992,9 @@ int lsd_ozaki_setup(lsd_ctx* ctx) {
     if (oz_prep_smem<OZ_ST>(o->srow[1]) > 200 * 1024 || oz_prep_smem<OZ_VEC>(o->srow[0]) > 200 * 1024)
       return lsd_fail(ctx, LSD_EARG, "tensor-core path: pre-pass rows do not fit in shared memory");
   }
+  CUDA_TRY(cudaMalloc(&o->d_err, sizeof(int)));
+  CUDA_TRY(cudaMemsetAsync(o->d_err, 0, sizeof(int), ctx->stream));
+  if (!lsd_ozaki_use_synth(ctx) && !lsd_ozaki_use_anal(ctx)) return LSD_OK;  // no tables, no digit buffers
   if (kidx.empty()) kidx.push_back(0);
   if (nhl.empty()) nhl.push_back(0);
   CUDA_TRY(cudaMalloc(&o->d_probs, sizeof(OzProb) * probs.size()));
@@ -991,8 +1017,6 @@ int lsd_ozaki_setup(lsd_ctx* ctx) {
     CUDA_TRY(cudaMalloc(&o->d_A[b], ab));
     CUDA_TRY(cudaMalloc(&o->d_erow[b], sizeof(int) * (size_t)NM * rows));
   }
-  CUDA_TRY(cudaMalloc(&o->d_err, sizeof(int)));
-  CUDA_TRY(cudaMemsetAsync(o->d_err, 0, sizeof(int), ctx->stream));
   OzTabArgs ta;
   ta.leg = ctx->d_leg; ta.H = ctx->H; ta.Th2 = Th2; ta.S = S; ta.NM = NM;
   ta.probs = o->d_probs; ta.kidx = o->d_kidx; ta.nhlist = o->d_nh; ta.B = o->d_B; ta.fexp = o->d_fexp;
@@ -1042,24 +1066,14 @@ int oz_run(lsd_ctx* ctx, const OzLaunchGroup* gs, int ng, cudaStream_t stream) {
   const dim3 pg(ctx->NM, nzb);
   const int srow = o->srow[OzT<TYPE>::anal ? 1 : 0];
   const size_t psm = oz_prep_smem<TYPE>(srow);
-  auto go = [&](auto kern) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm);
-    kern<<<pg, 256, psm, stream>>>(pa, srow);
-  };
-  switch (o->S) {
-    case 2: go(k_oz_prep<TYPE, 2>); break;
-    case 3: go(k_oz_prep<TYPE, 3>); break;
-    case 4: go(k_oz_prep<TYPE, 4>); break;
-    case 5: go(k_oz_prep<TYPE, 5>); break;
-    case 6: go(k_oz_prep<TYPE, 6>); break;
-    case 7: go(k_oz_prep<TYPE, 7>); break;
-    default: go(k_oz_prep<TYPE, 8>); break;
-  }
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->dev);
   const int ntile = ctx->NM * 2 * nzb;
-  oz_gemm_dispatch<TYPE>(o->S, [&](auto kern) {
-    kern<<<std::min(ntile, o->ctas * nsm), OZ_THREADS, o->smem, stream>>>(ga, nzb);
+  oz_slices_dispatch<TYPE>(o->S, [&](auto sc) {
+    constexpr int S = decltype(sc)::value;
+    cudaFuncSetAttribute(k_oz_prep<TYPE, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm);
+    k_oz_prep<TYPE, S><<<pg, 256, psm, stream>>>(pa, srow);
+    k_oz_gemm<TYPE, S><<<std::min(ntile, o->ctas * nsm), OZ_THREADS, o->smem, stream>>>(ga, nzb);
   });
   ctx->launches += 2;
   cudaError_t e = cudaGetLastError();

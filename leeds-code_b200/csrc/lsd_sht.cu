@@ -317,7 +317,7 @@ int launch_leg(lsd_ctx* ctx, LegBuilder& b) {
 }  // namespace
 
 int lsd_launch_synth(lsd_ctx* ctx, const SynthGroup* groups, int ngroups) {
-  if (ctx->oz) return lsd_ozaki_launch_synth(ctx, groups, ngroups);  // LSD_PREC_OZAKI
+  if (lsd_ozaki_use_synth(ctx)) return lsd_ozaki_launch_synth(ctx, groups, ngroups);
   LegBuilder b;
   bool ok = true;
   auto scalar = [&](const cplx* in, cplx* out, int tab, int flip, int rot, int scale) {
@@ -342,7 +342,7 @@ int lsd_launch_synth(lsd_ctx* ctx, const SynthGroup* groups, int ngroups) {
 }
 
 int lsd_launch_anal(lsd_ctx* ctx, const AnalGroup* groups, int ngroups) {
-  if (ctx->oz) return lsd_ozaki_launch_anal(ctx, groups, ngroups);  // LSD_PREC_OZAKI
+  if (lsd_ozaki_use_anal(ctx)) return lsd_ozaki_launch_anal(ctx, groups, ngroups);
   if (ceil_div(ctx->Hr, 32) * 32 > 1024) return lsd_fail(ctx, LSD_EARG, "analysis: folded column longer than 1024 harmonics");
   LegBuilder b;
   bool ok = true;

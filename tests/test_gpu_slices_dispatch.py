@@ -1,0 +1,53 @@
+"""LSD_PREC_OZAKI contexts on either side of the line between the int8-slice contraction and the
+FP64 tensor instruction (int8: up to 5 slices, and the analysis at 6 above L = 192): every
+transform against the oracle, with odd theta counts and partial tiles.
+
+Tolerance: S slices carry 8 S - 2 bits of each operand's row or column maximum; the measured errors
+at lmax 127 are 2.9e-9 (S = 5), 1.4e-11 (6), 9.6e-7 (4) and 256 times that per slice less, of the largest
+output; the bounds leave 4 times 256^(5 - S) 5e-9.  Where the FP64 instruction runs: 1e-12.
+"""
+import importlib
+
+import numpy as np
+import pytest
+
+import oracle_lib as ol
+
+pkg = importlib.import_module("leeds-code_b200")
+capi = pkg.capi
+
+
+def relerr(a, b):
+    return float(np.abs(np.asarray(a) - np.asarray(b)).max() / max(np.abs(np.asarray(b)).max(), 1e-300))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,M,S", [(17, 8, 2), (79, 64, 3), (113, 64, 4), (128, 16, 5), (33, 32, 6), (192, 32, 6),
+                                   (193, 32, 6), (200, 64, 6), (200, 64, 7), (64, 64, 8)])
+def test_transforms_across_the_dispatch(L, M, S):
+    kw = dict(L=L, M=M, Mp=1, N=7, KL=2, timestep=1e-5)
+    g, o = pkg.Context(capi.template_config(precision=capi.PREC_OZAKI, ozaki_slices=S, **kw)), ol.Oracle(
+        capi.template_config(**kw))
+    slices = 4 * 256.0 ** (5 - S) * 5e-9
+    tol_s = slices if S <= 5 else 1e-12
+    tol_a = slices if S <= 5 or (S == 6 and L > 192) else 1e-12
+    rng = np.random.default_rng(L + M + S)
+    _, m, _ = o.harmonics()
+
+    def spec():
+        re, im = rng.standard_normal((2, o.N, o.H))
+        im[:, m == 0] = 0
+        return re, im
+
+    q, s, t = spec(), spec(), spec()
+    grid = [rng.standard_normal((o.N, o.Ph, o.Th)) for _ in range(3)]
+    assert relerr(g.tra_spec2phys(*q), o.spec2phys(*q)) < tol_s
+    for x, y in zip(g.tra_qst2rtp(q, s, t), o.qst2rtp(q, s, t)):
+        assert relerr(x, y) < tol_s
+    for x, y in zip(g.tra_grad(*q), o.grad(*q)):
+        assert relerr(x, y) < tol_s
+    assert relerr(g.tra_phys2spec(grid[0]), o.phys2spec(grid[0])) < tol_a
+    for x, y in zip(g.tra_rtp2qst(*grid), o.rtp2qst(*grid)):
+        assert relerr(x, y) < tol_a
+    g.close()
+    o.close()
