@@ -43,7 +43,7 @@ void free_ctx(lsd_ctx* ctx) {
                   ctx->d_leg, ctx->d_gp, ctx->d_gw, ctx->d_sn, ctx->d_sn1, ctx->d_tw2, ctx->d_twh, ctx->d_r,
                   ctx->d_dr, ctx->d_r1dr, ctx->d_radlap, ctx->d_intr2dr, ctx->d_lu, ctx->d_y, ctx->d_lf, ctx->d_uf, ctx->d_yf,
                   ctx->d_ipiv, ctx->d_info, ctx->d_gf, ctx->d_invg, ctx->d_state, ctx->d_nl,
-                  ctx->d_sv, ctx->d_spec, ctx->d_four, ctx->d_phys, ctx->d_red, ctx->d_cpart, ctx->d_ref, ctx->d_laps,
+                  ctx->d_sv, ctx->d_spec, ctx->d_four, ctx->d_phys, ctx->d_red, ctx->d_epack, ctx->d_cpart, ctx->d_ref, ctx->d_laps,
                   ctx->d_compr1dr, ctx->d_wts, ctx->d_ones, ctx->d_cfl, ctx->d_icr, ctx->d_icdr, ctx->d_icradlap,
                   ctx->d_icr1dr, ctx->d_icintr2dr, ctx->d_icwts, ctx->d_icref, ctx->d_iclaps, ctx->d_iccompr1dr,
                   ctx->d_icyf, ctx->d_icstate, ctx->d_icsv, ctx->d_rot, ctx->d_gwP0, ctx->d_grescr,
@@ -703,6 +703,7 @@ int lsd_create(const lsd_config* cfg, lsd_ctx** out) {
   }
   TRY(dalloc(ctx, &ctx->d_four, (size_t)ctx->nfour * N * ctx->HB * NM * 4));
   TRY(dalloc(ctx, &ctx->d_red, (size_t)128 + 48 * N));
+  TRY(dalloc(ctx, &ctx->d_epack, (size_t)(21 + 2 * KL) * N + 6));
   TRY(dalloc(ctx, &ctx->d_cpart, (size_t)8 * nlb * c.M));
   TRY(dalloc(ctx, &ctx->d_cfl, (size_t)2 * N + 1));
   CTRY(cudaMallocHost((void**)&ctx->h_red, sizeof(double) * 64));

@@ -172,6 +172,7 @@ struct lsd_ctx {
   size_t h_pin_bytes = 0;
   // reductions
   double *d_red = nullptr;   // small reduction area
+  double *d_epack = nullptr; // what the energies' radial sums need, gathered for one copy (k_energy_pack)
   double *d_cpart = nullptr; // corrector: per-warp sums of squares [8][nlb][M]
   double *h_red = nullptr;   // pinned mirror (64 doubles; slots below)
   // time

@@ -491,17 +491,21 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 2) k_step_solves(StepArgs a) {
 
 // rot_predictor / rot_corrector (rotation.F90:40-87) with the torques of non_rotation
 // (nonlinear.F90:479-538) from k_products' surface sums (np half-rows' pairs after the
-// ROT_NSLOT slots, added here in order); one thread.  The rate of the evaluation is kept
+// ROT_NSLOT slots, added here in a fixed order: lanes in strides of 32, then a tree); one warp.  The rate of the evaluation is kept
 // for the inner core's nonlinear term of the solves that follow.
 __global__ void k_rot(double* rot, int np, int corr, double inertia, double implicit, double Ph, double vfac,
                       double mfac, int vel_on, int mag_on, int force0) {
-  if (threadIdx.x != 0) return;
   const double PI = 3.1415926535897931;
   double sv = 0.0, sm = 0.0;
-  for (int h = 0; h < np; ++h) {
+  for (int h = threadIdx.x; h < np; h += 32) {
     sv = sv + rot[ROT_NSLOT + 2 * h];
     sm = sm + rot[ROT_NSLOT + 2 * h + 1];
   }
+  for (int o = 16; o > 0; o >>= 1) {
+    sv += __shfl_down_sync(0xffffffffu, sv, o);
+    sm += __shfl_down_sync(0xffffffffu, sm, o);
+  }
+  if (threadIdx.x != 0) return;
   rot[ROT_SUM_VEL] = sv;
   rot[ROT_SUM_MAG] = sm;
   rot[ROT_OMEGA_EVAL] = rot[ROT_OMEGA];
@@ -562,10 +566,11 @@ __global__ void __launch_bounds__(32) k_greens(int N, int NL, int L, int nlb, co
 // fixed tree, so the sums (and every diagnostic built on them) are the same bits on every
 // call for the same state.
 constexpr int NORM_THREADS = 256;
-__global__ void __launch_bounds__(NORM_THREADS) k_norms(int N, int H, const int* hl, const int* hm,
-                                                        const cplx* const* arrs, double* out) {
+struct NormArgs { const cplx* a[12]; };
+__global__ void __launch_bounds__(NORM_THREADS) k_norms(int N, int H, const int* hl, const int* hm, NormArgs arrs,
+                                                        double* out) {
   const int n = blockIdx.x, k = blockIdx.y;
-  const double2* a = arrs[k] + (size_t)n * H;
+  const double2* a = arrs.a[k] + (size_t)n * H;
   double c[4] = {0.0, 0.0, 0.0, 0.0};
   for (int nh = threadIdx.x; nh < H; nh += NORM_THREADS) {
     const int l = hl[nh], m_ = hm[nh];
@@ -868,13 +873,35 @@ int lsd_corr(lsd_ctx* ctx) {
 
 namespace {
 
+// What the host's radial sums need besides the norms, gathered by one kernel and copied at once (eight
+// copies from pageable memory took 140 us of a call): wts 5 N (intr2dr, intr2dr_comp, _compS, _magdiss,
+// _veldiss), the codensity's l = 0 column N, r 7 N, ref 7 N, dr(1)'s band (2 KL + 1) N, the first three
+// poloidal field coefficients at r_o.
+__global__ void k_energy_pack(int N, int H, int KL, const double* intr2dr, const double* wts, const cplx* cod,
+                              const double* r, const double* ref, const double* dr1, const cplx* bpol, double* out) {
+  const int W = 20 + 2 * KL + 1;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < W * N + 6; i += gridDim.x * blockDim.x) {
+    const int k = i / N, n = i - k * N;
+    double v;
+    if (k == 0) v = intr2dr[n];
+    else if (k < 5) v = wts[(size_t)(k - 1) * N + n];
+    else if (k == 5) v = cod[(size_t)n * H].x;
+    else if (k < 13) v = r[(size_t)(k - 6) * N + n];
+    else if (k < 20) v = ref[(size_t)(k - 13) * N + n];
+    else if (i < W * N) v = dr1[i - 20 * N];
+    else v = ((const double*)(bpol + (size_t)(N - 1) * H))[i - W * N];
+    out[i] = v;
+  }
+}
+
+// the host's view of one call's norms and of k_energy_pack's gather, in the pinned staging buffer
+struct EnergyHost { const double *Fh, *wts, *cod0, *r, *ref, *dr1, *bpolN; };
+
 // The derived fields (q, s, t and curl of velocity and field), their per-(field,
 // category, shell) norms written to d_out (48 N doubles; k_norms writes every slot once,
 // each a fixed-order tree sum, so nothing needs clearing), and host copies of all that
-// the radial sums need.  d_arrs: device room for 12 pointers.
-// wts: 5 N (intr2dr, intr2dr_comp, _compS, _magdiss, _veldiss), ref: 7 N.
-int energy_partials(lsd_ctx* ctx, const cplx** d_arrs, double* d_out, double* Fh, double* wts, double* cod0,
-                    double* bpolN, double* r, double* dr1, double* ref) {
+// the radial sums need.
+int energy_partials(lsd_ctx* ctx, double* d_out, EnergyHost* h) {
   const int N = ctx->N, H = ctx->H, KL = ctx->KL;
   const size_t F = (size_t)N * H;
   cplx* sp = ctx->d_spec;
@@ -889,22 +916,26 @@ int energy_partials(lsd_ctx* ctx, const cplx** d_arrs, double* d_out, double* Fh
   k_qst<<<g, 128, 0, s>>>(sa, ctx->d_r1dr, st + LSD_MAG_TOR * F, st + LSD_MAG_POL * F, sp + 6 * F, sp + 7 * F,
                           sp + 8 * F);
   k_curl<<<g, 128, 0, s>>>(sa, sp + 6 * F, sp + 7 * F, sp + 8 * F, sp + 9 * F, sp + 10 * F, sp + 11 * F);
-  const cplx* arrs[12];
-  for (int k = 0; k < 12; ++k) arrs[k] = sp + k * F;
-  CUDA_TRY(cudaMemcpyAsync(d_arrs, arrs, sizeof(arrs), cudaMemcpyHostToDevice, s));
-  k_norms<<<dim3(N, 12), NORM_THREADS, 0, s>>>(N, H, ctx->d_l, ctx->d_m, d_arrs, d_out);
-  ctx->launches += 5;
-  CUDA_TRY(cudaMemcpyAsync(Fh, d_out, sizeof(double) * 48 * N, cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(cudaMemcpyAsync(wts, ctx->d_intr2dr, sizeof(double) * N, cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(cudaMemcpyAsync(wts + N, ctx->d_wts, sizeof(double) * 4 * N, cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(cudaMemcpyAsync(ref, ctx->d_ref, sizeof(double) * 7 * N, cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(cudaMemcpyAsync(r, ctx->d_r, sizeof(double) * 7 * N, cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(cudaMemcpyAsync(dr1, ctx->d_dr, sizeof(double) * (2 * KL + 1) * N, cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(cudaMemcpy2DAsync(cod0, sizeof(double), st + LSD_COD_C * F, sizeof(cplx) * H, sizeof(double), N,
-                             cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(cudaMemcpyAsync(bpolN, st + LSD_MAG_POL * F + (size_t)(N - 1) * H, sizeof(cplx) * 3,
-                           cudaMemcpyDeviceToHost, s));
+  NormArgs arrs;
+  for (int k = 0; k < 12; ++k) arrs.a[k] = sp + k * F;
+  k_norms<<<dim3(N, 12), NORM_THREADS, 0, s>>>(N, H, ctx->d_l, ctx->d_m, arrs, d_out);
+  const int W = 20 + 2 * KL + 1, total = W * N + 6;
+  k_energy_pack<<<std::min(ceil_div(total, 256), 148), 256, 0, s>>>(
+      N, H, KL, ctx->d_intr2dr, ctx->d_wts, st + LSD_COD_C * F, ctx->d_r, ctx->d_ref, ctx->d_dr, st + LSD_MAG_POL * F,
+      ctx->d_epack);
+  ctx->launches += 6;
+  CUDA_TRY(cudaGetLastError());
+  double* p = ctx->h_pin;
+  CUDA_TRY(cudaMemcpyAsync(p, d_out, sizeof(double) * 48 * N, cudaMemcpyDeviceToHost, s));
+  CUDA_TRY(cudaMemcpyAsync(p + 48 * N, ctx->d_epack, sizeof(double) * total, cudaMemcpyDeviceToHost, s));
   CUDA_TRY(cudaStreamSynchronize(s));
+  h->Fh = p;
+  h->wts = p + (size_t)48 * N;
+  h->cod0 = h->wts + (size_t)5 * N;
+  h->r = h->cod0 + N;
+  h->ref = h->r + (size_t)7 * N;
+  h->dr1 = h->ref + (size_t)7 * N;
+  h->bpolN = h->dr1 + (size_t)(2 * KL + 1) * N;
   return LSD_OK;
 }
 
@@ -996,13 +1027,10 @@ int energy_finish(lsd_ctx* ctx, const double* Fh, const double* wts, const doubl
 // Energy diagnostics (io_write_vel_energy io.F90:1739-1926, io_write_mag_energy
 // io.F90:1933-2024): device norms, host radial dot products in the reference's order.
 int lsd_energy_device(lsd_ctx* ctx, double* out) {
-  const int N = ctx->N, KL = ctx->KL;
-  std::vector<double> Fh((size_t)48 * N), wts(5 * N), cod0(N), bpolN(3 * 2), r(N * 7), dr1((size_t)(2 * KL + 1) * N),
-      ref(7 * N);
-  int rc = energy_partials(ctx, (const cplx**)(ctx->d_red + 64), ctx->d_red + 128, Fh.data(), wts.data(),
-                           cod0.data(), bpolN.data(), r.data(), dr1.data(), ref.data());
+  EnergyHost h;
+  int rc = energy_partials(ctx, ctx->d_red + 128, &h);
   if (rc) return rc;
-  return energy_finish(ctx, Fh.data(), wts.data(), cod0.data(), bpolN.data(), r.data(), dr1.data(), ref.data(), out);
+  return energy_finish(ctx, h.Fh, h.wts, h.cod0, h.bpolN, h.r, h.dr1, h.ref, out);
 }
 
 // ---- energies with no allocation -------------------------------------------------------
@@ -1010,8 +1038,8 @@ int lsd_energy_device(lsd_ctx* ctx, double* out) {
 // when they ask for diagnostics -- a host code whose device memory is fully committed to
 // its state arrays (cudaMalloc would fail), or one that keeps work queued on its stream
 // while it writes output (cudaMalloc / cudaFree synchronise the device and would stall that
-// pipeline).  The norm partial sums and the 12 field pointers live in a file-scope device
-// array instead of context memory; host staging uses the context's pinned buffer, which
+// pipeline).  The norm partial sums live in a file-scope device array instead of context
+// memory; host staging uses the context's pinned buffer, which
 // lsd_create sizes for it.  The norm kernel writes every slot of the array once per call
 // (a fixed-order tree sum per slot, no atomics), so the previous call's contents are
 // simply overwritten and nothing is cleared.  The array is shared by every context on a
@@ -1021,9 +1049,8 @@ int lsd_energy_device(lsd_ctx* ctx, double* out) {
 // process may load this module, so make the first call before any stream capture).
 namespace {
 constexpr int ESTATIC_MAX_N = 1024;  // shells
-constexpr int ESTATIC_PTRS = 16;     // 12 field pointers, padded to 128 bytes
 }  // namespace
-static __device__ __align__(256) double g_energy_scratch[ESTATIC_PTRS + 48 * ESTATIC_MAX_N];  // 384 KiB + 128 B
+static __device__ __align__(256) double g_energy_scratch[48 * ESTATIC_MAX_N];  // 384 KiB
 
 int lsd_energy_static(lsd_ctx* ctx, double* out) {
   const int N = ctx->N, KL = ctx->KL;
@@ -1044,16 +1071,10 @@ int lsd_energy_static(lsd_ctx* ctx, double* out) {
       return lsd_fail(ctx, LSD_ECUDA, msg);
     }
   }
-  double* Fh = ctx->h_pin;
-  double* wts = Fh + (size_t)48 * N;
-  double* cod0 = wts + (size_t)5 * N;
-  double* bpolN = cod0 + N;
-  double* r = bpolN + 6;
-  double* dr1 = r + (size_t)7 * N;
-  double* ref = dr1 + (size_t)(2 * KL + 1) * N;
-  int rc = energy_partials(ctx, (const cplx**)dscr, dscr + ESTATIC_PTRS, Fh, wts, cod0, bpolN, r, dr1, ref);
+  EnergyHost h;
+  int rc = energy_partials(ctx, dscr, &h);
   if (rc) return rc;
-  return energy_finish(ctx, Fh, wts, cod0, bpolN, r, dr1, ref, out);
+  return energy_finish(ctx, h.Fh, h.wts, h.cod0, h.bpolN, h.r, h.dr1, h.ref, out);
 }
 
 // ---- the other diagnostics of io_write2files ------------------------------------------
@@ -1165,11 +1186,12 @@ int lsd_diagnostics_device(lsd_ctx* ctx, double* sc, double* spec, double* prof)
   cplx* st = ctx->d_state;
   cudaStream_t s = ctx->stream;
   // energies and the category norms of q, s, t (slots 0..11 of the spectral scratch)
-  std::vector<double> Fh((size_t)48 * N), wts(5 * N), cod0(N), bpolN(3 * 2), r(N * 7),
-      dr1((size_t)(2 * KL + 1) * N), ref(7 * N), en(LSD_NENERGY);
-  int rc = energy_partials(ctx, (const cplx**)(ctx->d_red + 64), ctx->d_red + 128, Fh.data(), wts.data(),
-                           cod0.data(), bpolN.data(), r.data(), dr1.data(), ref.data());
+  EnergyHost eh;
+  int rc = energy_partials(ctx, ctx->d_red + 128, &eh);
   if (rc) return rc;
+  std::vector<double> Fh(eh.Fh, eh.Fh + (size_t)48 * N), wts(eh.wts, eh.wts + (size_t)5 * N),
+      cod0(eh.cod0, eh.cod0 + N), bpolN(eh.bpolN, eh.bpolN + 6), r(eh.r, eh.r + (size_t)7 * N),
+      dr1(eh.dr1, eh.dr1 + (size_t)(2 * KL + 1) * N), ref(eh.ref, eh.ref + (size_t)7 * N), en(LSD_NENERGY);
   if ((rc = energy_finish(ctx, Fh.data(), wts.data(), cod0.data(), bpolN.data(), r.data(), dr1.data(), ref.data(),
                           en.data())))
     return rc;
@@ -1284,12 +1306,10 @@ int lsd_diagnostics_device(lsd_ctx* ctx, double* sc, double* spec, double* prof)
     dim3 gi(ceil_div(H, 128), Ni);
     k_qst<<<gi, 128, 0, s>>>(si, ctx->d_icr1dr, ctx->d_icstate, ctx->d_icstate + Fi, sp, sp + F, sp + 2 * F);
     k_curl<<<gi, 128, 0, s>>>(si, sp, sp + F, sp + 2 * F, sp + 3 * F, sp + 4 * F, sp + 5 * F);
-    const cplx* arrs[6];
-    for (int k = 0; k < 6; ++k) arrs[k] = sp + k * F;
-    const cplx** d_arrs = (const cplx**)(ctx->d_red + 64);
+    NormArgs arrs{};
+    for (int k = 0; k < 6; ++k) arrs.a[k] = sp + k * F;
     double* d_out = ctx->d_red + 128;
-    CUDA_TRY(cudaMemcpyAsync(d_arrs, arrs, sizeof(arrs), cudaMemcpyHostToDevice, s));
-    k_norms<<<dim3(Ni, 6), NORM_THREADS, 0, s>>>(Ni, H, ctx->d_l, ctx->d_m, d_arrs, d_out);
+    k_norms<<<dim3(Ni, 6), NORM_THREADS, 0, s>>>(Ni, H, ctx->d_l, ctx->d_m, arrs, d_out);
     ctx->launches += 3;
     std::vector<double> Fi_h((size_t)24 * Ni), wic((size_t)5 * Ni);
     CUDA_TRY(cudaMemcpyAsync(Fi_h.data(), d_out, sizeof(double) * Fi_h.size(), cudaMemcpyDeviceToHost, s));
