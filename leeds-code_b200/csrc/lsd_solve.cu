@@ -855,7 +855,7 @@ int lsd_pred(lsd_ctx* ctx) {
   if (rc) return rc;
   ctx->launches++;
   cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return lsd_fail(ctx, LSD_ECUDA, std::string("k_predictor: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) return lsd_fail(ctx, LSD_ECUDA, std::string("k_step_solves: ") + cudaGetErrorString(e));
   return LSD_OK;
 }
 
@@ -867,7 +867,7 @@ int lsd_corr(lsd_ctx* ctx) {
   k_cgce_sums<<<1, 256, 0, ctx->stream>>>(ctx->d_cpart, a.nwarp, ctx->d_red);
   ctx->launches += 2;
   cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return lsd_fail(ctx, LSD_ECUDA, std::string("k_corrector: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) return lsd_fail(ctx, LSD_ECUDA, std::string("k_step_solves: ") + cudaGetErrorString(e));
   return LSD_OK;
 }
 
