@@ -70,8 +70,9 @@ extern "C" {
 /* precision of the Legendre contraction */
 #define LSD_PREC_FP64   0   /* FP64 products and sums (the FP64 tensor instruction)      */
 #define LSD_PREC_OZAKI  1   /* at least the precision of ozaki_slices int8 slices: the slices
-                               on the tcgen05 tensor cores (up to five), from six on FP64
-                               where that is faster (all but large analyses at six)      */
+                               on the tcgen05 tensor cores (up to five, and eight), at six
+                               and seven FP64 where that is faster (all but large analyses
+                               at six)                                                   */
 
 /* energy diagnostics written by lsd_energies (io.F90:1739-2024 column order) */
 #define LSD_E_TIME     0   /* tim_t                                                      */
@@ -134,8 +135,9 @@ typedef struct lsd_config {
   int precision;            /* LSD_PREC_* for the Legendre contraction                */
   int device;               /* CUDA device ordinal                                    */
   int ozaki_slices;         /* int8 slices per operand for LSD_PREC_OZAKI, 2..8 (0 = 7):
-                               S balanced base-256 digits carry 8S - 2 bits (rounded); 5
-                               keep 1000-step energies within ~1e-11 of FP64, 7 match FP64 */
+                               S balanced base-256 digits carry 8S - 2 bits (rounded) of a
+                               row or column maximum; 5 keep 1000-step energies within ~1e-11
+                               of FP64, 6 and 7 run as FP64 where that is faster, 8 exceed it */
   /* physics (parameters.F90_template:29-44) */
   double rratio, alpha, Ra, Ra_comp, Pr, Sc, Pm, E, Hyp;
   /* time integration (parameters.F90_template:229-243) */

@@ -847,6 +847,7 @@ void oz_slices_dispatch(int S, F&& f) {
     case 4: f(std::integral_constant<int, 4>()); break;
     case 5: f(std::integral_constant<int, 5>()); break;
     case 6: if constexpr (OzT<TYPE>::anal) f(std::integral_constant<int, 6>()); break;
+    case 8: f(std::integral_constant<int, 8>()); break;
     default: break;
   }
 }
@@ -870,14 +871,17 @@ void oz_set_smem(int S, size_t smem) {
 // From six slices on the S (S + 1) / 2 digit products and the slicing pass cost more than the FP64
 // products at every size but one: six slices in the analysis above L = 192, whose slicing pass over
 // the theta rows is spread over the most harmonics.  Up to five slices the int8 path stays at all
-// sizes: a caller who asked for 38 bits gets the rounding of 38 bits.
+// sizes: a caller who asked for 38 bits gets the rounding of 38 bits.  Eight slices stay on int8 for
+// their precision, 62 bits of each row or column maximum and exact digit sums: sums of 32 products that
+// rise to 5 to 16 times their value and fall are off by 9.8e-18 of the largest (RMS, against exact
+// fractions), a chain of FP64 multiply-adds by 5.5e-17, seven slices by 3.0e-16, six by 7.4e-14.
 bool lsd_ozaki_use_synth(const lsd_ctx* c) {
   const OzState* o = (const OzState*)c->oz;
-  return o && o->S <= 5;
+  return o && (o->S <= 5 || o->S == 8);
 }
 bool lsd_ozaki_use_anal(const lsd_ctx* c) {
   const OzState* o = (const OzState*)c->oz;
-  return o && (o->S <= 5 || (o->S == 6 && c->L > 192));
+  return o && (o->S <= 5 || o->S == 8 || (o->S == 6 && c->L > 192));
 }
 
 void lsd_ozaki_free(lsd_ctx* ctx) {

@@ -7,6 +7,7 @@ at lmax 127 are 2.9e-9 (S = 5), 1.4e-11 (6), 9.6e-7 (4) and 256 times that per s
 output; the bounds leave 4 times 256^(5 - S) 5e-9.  Where the FP64 instruction runs: 1e-12.
 """
 import importlib
+from fractions import Fraction
 
 import numpy as np
 import pytest
@@ -51,3 +52,48 @@ def test_transforms_across_the_dispatch(L, M, S):
         assert relerr(x, y) < tol_a
     g.close()
     o.close()
+
+
+@pytest.mark.gpu
+def test_eight_slices_exceed_fp64():
+    """Eight slices carry 62 bits of the power of two above each operand's row or column maximum and
+    sum digit products exactly; the diagonals are joined by Horner's rule in FP64, whose last two
+    steps exceed 53 bits.  A sum of K products is off by at most 2 x 2^-53 |sum| for these two
+    roundings, K (2 x 2^-63 + 9 x 2^-62) of the powers' product for the operands' rounding and the
+    dropped digit pairs, and 2^-53 K / 60 of it for the part of the lower diagonals in the sums that
+    are rounded.  A chain of FP64 multiply-adds exceeds that here, where the partial sums are far
+    larger than the sum.  The phi transform is exact for these inputs: m = 0 alone,
+    and a grid with one phi sample."""
+    L, M, N = 64, 16, 7
+    g = pkg.Context(capi.template_config(L=L, M=M, Mp=1, N=N, KL=2, timestep=1e-5, precision=capi.PREC_OZAKI,
+                                         ozaki_slices=8))
+    rng = np.random.default_rng(8)
+    l, m, _ = g.harmonics()
+
+    def rise_and_fall(k):
+        return np.where(np.arange(k) < k // 2, 1.0, -1.0) * (0.99 - 0.25 * rng.random((N, k)))
+
+    def check(got, c, T):  # got[n, i] = sum_k c[n, k] T[i, k]
+        a = c.shape[1] * (10.0 / 512.0 + 1.0 / 60.0)
+        cf = [[Fraction(v) for v in row] for row in c.tolist()]
+        above = lambda v: 2.0 ** int(np.frexp(np.abs(v).max())[1])
+        for i, row in enumerate(T.tolist()):
+            tf = [Fraction(v) for v in row]
+            for n in range(N):
+                x = sum(u * v for u, v in zip(cf[n], tf))
+                err = abs(float(Fraction(float(got[n, i])) - x))
+                assert err <= 2.0 ** -53 * (2.0 * abs(float(x)) + a * above(c[n]) * above(T[i])), (n, i)
+
+    idx = np.flatnonzero((m == 0) & (l % 2 == 0))
+    re, im = np.zeros((2, N, g.H))
+    re[:, idx] = rise_and_fall(idx.size)
+    phys = g.tra_spec2phys(re, im)
+    assert np.array_equal(phys, np.broadcast_to(phys[:, :1, :], phys.shape))
+    check(phys[:, 0, :g.Th2], re[:, idx], g.legendre_table(capi.LEG_P)[:, idx])
+
+    grid = np.zeros((N, g.Ph, g.Th))
+    grid[:, 0, :g.Th2] = rise_and_fall(g.Th2)
+    re, im = g.tra_phys2spec(grid)
+    idx = np.flatnonzero(m == 0)
+    check(re[:, idx], grid[:, 0, :g.Th2] * (1.0 / g.Ph), g.legendre_table(capi.LEG_GWP)[:, idx].T)
+    g.close()
