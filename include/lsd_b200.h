@@ -71,8 +71,7 @@ extern "C" {
 #define LSD_PREC_FP64   0   /* FP64 products and sums (the FP64 tensor instruction)      */
 #define LSD_PREC_OZAKI  1   /* at least the precision of ozaki_slices int8 slices: the slices
                                on the tcgen05 tensor cores (up to five, and eight), at six
-                               and seven FP64 where that is faster (all but large analyses
-                               at six)                                                   */
+                               and seven FP64 where that is faster (small L, or M near L) */
 
 /* energy diagnostics written by lsd_energies (io.F90:1739-2024 column order) */
 #define LSD_E_TIME     0   /* tim_t                                                      */

@@ -805,6 +805,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 2) k_oz_gemm(OzGemmArgs a, int nzb
 // =========================================================================================
 struct OzState {
   int S = 0;
+  bool synth = false, anal = false;  // the direction runs on the slices (oz_route)
   int nzb_max[OZ_NTYPE] = {};
   OzProb* d_probs = nullptr;
   int* d_kidx = nullptr;
@@ -837,8 +838,7 @@ constexpr int OZ_MAXG_SYNTH = OZ_MAXG, OZ_MAXG_ANAL = 4;  // groups per launch
 // the digit / exponent buffer of each type's chain
 int oz_buf(int type) { return type == OZ_VEC || type == OZ_ST ? 0 : type == OZ_P || type == OZ_Q ? 1 : 2; }
 
-// f(integral_constant S) for the runtime slice count S; nothing for the counts at which the type's
-// contractions run on the FP64 instruction (lsd_ozaki_use_synth / _anal)
+// f(integral_constant S) for the runtime slice count S
 template <int TYPE, class F>
 void oz_slices_dispatch(int S, F&& f) {
   switch (S) {
@@ -846,7 +846,8 @@ void oz_slices_dispatch(int S, F&& f) {
     case 3: f(std::integral_constant<int, 3>()); break;
     case 4: f(std::integral_constant<int, 4>()); break;
     case 5: f(std::integral_constant<int, 5>()); break;
-    case 6: if constexpr (OzT<TYPE>::anal) f(std::integral_constant<int, 6>()); break;
+    case 6: f(std::integral_constant<int, 6>()); break;
+    case 7: f(std::integral_constant<int, 7>()); break;
     case 8: f(std::integral_constant<int, 8>()); break;
     default: break;
   }
@@ -868,20 +869,39 @@ void oz_set_smem(int S, size_t smem) {
 //   128, 129   471 + 301    411 + 266   430 + 277   451 + 289   494 + 307   555 + 320   666 + 344
 //   192, 97   1055 + 602    935 + 494   970 + 516  1084 + 547  1153 + 602  1235 + 641  1452 + 721
 //   256, 65   1569 + 917   1448 + 596  1563 + 648  1657 + 707  1737 + 787  2029 + 871  2268 + 989
-// From six slices on the S (S + 1) / 2 digit products and the slicing pass cost more than the FP64
-// products at every size but one: six slices in the analysis above L = 192, whose slicing pass over
-// the theta rows is spread over the most harmonics.  Up to five slices the int8 path stays at all
-// sizes: a caller who asked for 38 bits gets the rounding of 38 bits.  Eight slices stay on int8 for
+// (FP64 at every L = M from six slices on, but for the analysis of 256 at six).
+//
+// Six and seven slices take the faster side.  The digit products grow with S (S + 1) / 2 and the
+// slicing pass is paid per order and value, so int8 gains with K, the mean number of harmonics per
+// order; the FP64 contraction pays for theta rows padded to tiles of 48 (synthesis, a factor pad) and for
+// the 8-byte table copies of an odd half grid (15 %, odd).  FP64 / int8 measured at 62 shapes (L 64 .. 264,
+// M 12 .. 256, Mp 1 .. 12, N 20 .. 99; the geometric mean in brackets):
+//   synthesis  S = 6: K pad odd <= 122 0.40 .. 1.06 (0.67), up to 152 0.86 .. 1.18 (0.98), above 0.76 .. 1.50 (1.11)
+//              S = 7:           <= 175 0.39 .. 0.99 (0.72), up to 219 0.70 .. 1.25 (0.93), above 0.69 .. 1.26 (0.99)
+//   analysis   S = 6: K odd     <= 124 0.47 .. 1.06 (0.76), up to 155 0.61 .. 1.15 (0.99), above 0.70 .. 1.44 (1.06)
+//              S = 7:           <= 160 0.46 .. 1.02 (0.77), up to 200 0.65 .. 1.08 (0.90), above 0.73 .. 1.25 (1.00)
+// Beyond the bounds int8 also keeps shapes of few columns (M = 16, N = 33), where FP64 would win.
+// Up to five slices int8 stays at all sizes, though FP64 is faster at most of them: it would move the
+// outputs of such a run by the slices' own rounding (two steps of an anelastic member at five slices by
+// 1.9e-10 of the largest coefficient).  Eight slices stay for
 // their precision, 62 bits of each row or column maximum and exact digit sums: sums of 32 products that
 // rise to 5 to 16 times their value and fall are off by 9.8e-18 of the largest (RMS, against exact
 // fractions), a chain of FP64 multiply-adds by 5.5e-17, seven slices by 3.0e-16, six by 7.4e-14.
+namespace {
+void oz_route(const lsd_ctx* c, OzState* o) {
+  const double K = (double)c->H / c->M * (c->Th2 & 1 ? 1.15 : 1.0), pad = 48.0 * ceil_div(c->Th2, 48) / c->Th2;
+  const int S = o->S;
+  o->synth = S <= 5 || S == 8 || K * pad > (S == 6 ? 122.0 : 175.0);
+  o->anal = S <= 5 || S == 8 || K > (S == 6 ? 124.0 : 160.0);
+}
+}  // namespace
 bool lsd_ozaki_use_synth(const lsd_ctx* c) {
   const OzState* o = (const OzState*)c->oz;
-  return o && (o->S <= 5 || o->S == 8);
+  return o && o->synth;
 }
 bool lsd_ozaki_use_anal(const lsd_ctx* c) {
   const OzState* o = (const OzState*)c->oz;
-  return o && (o->S <= 5 || o->S == 8 || (o->S == 6 && c->L > 192));
+  return o && o->anal;
 }
 
 void lsd_ozaki_free(lsd_ctx* ctx) {
@@ -908,6 +928,7 @@ int lsd_ozaki_setup(lsd_ctx* ctx) {
   const int S = ctx->cfg.ozaki_slices > 0 ? ctx->cfg.ozaki_slices : 7;
   if (S < 2 || S > OZ_MAXS) return lsd_fail(ctx, LSD_EARG, "ozaki_slices must be 2..8");
   o->S = S;
+  oz_route(ctx, o);
   const int NM = ctx->NM, Th2 = ctx->Th2, N = ctx->N;
   for (int c = 0; c < NM; ++c)
     if (ctx->mlen[c] > 512) return lsd_fail(ctx, LSD_EARG, "tensor-core path: more than 512 harmonics per m");
