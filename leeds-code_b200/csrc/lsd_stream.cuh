@@ -18,8 +18,10 @@
 // way) and, with many columns, the instructions of a row.  So no load stands in the chain (a
 // row loaded when it is needed costs 0.7 us per batch of rows) and no division (114 cycles): x / d is
 // formed from the stored reciprocal with one correction step (Markstein, IBM J. Res. Dev. 34, 111
-// (1990): q = x r, then q + (x - q d) r, the rounded quotient when r is the rounded
-// reciprocal).  Sharing the factors between four orders takes their traffic from 84 to 21 bytes
+// (1990): q = x r, then q + (x - q d) r).  q is off by at most 2^-52 of itself and r by 2^-53 of itself,
+// so the sum before its rounding is off by 2^-105: the rounded quotient, but for quotients that close to a
+// tie, as long as r is a normal number (the factorisation multiplies by the same reciprocals) and
+// |x| is above 2^-968, where x - q d is exact.  Sharing the factors between four orders takes their traffic from 84 to 21 bytes
 // per column row and pass.  All passes of a column run through one copy of the code (a loop
 // over pass descriptors): with a copy per pass the short columns of a small run waited for
 // instruction fetches half of their time.
@@ -58,10 +60,11 @@ __device__ __forceinline__ void sv_cp16(void* dst, const void* src, int bytes) {
 __device__ __forceinline__ double2 axpy2(double2 y, double a, double2 x) {  // y + a x
   return make_double2(y.x + a * x.x, y.y + a * x.y);
 }
-// x / d from r = the rounded 1 / d
+// x / d from r = the rounded 1 / d.  An infinite or NaN x r stays as it is (inf / d = inf; the
+// correction would make it NaN); the select costs 0.7 % of a solve, a branch to a division 4 to 10 %.
 __device__ __forceinline__ double sv_div(double x, double d, double r) {
-  const double q = x * r;
-  return fma(fma(-q, d, x), r, q);
+  const double q = x * r, e = fma(-q, d, x);
+  return fma((__double2hiint(q) & 0x7fffffff) < 0x7ff00000 ? e : 0.0, r, q);
 }
 
 // One pass over the N rows of a system, a thread's column (row stride rst) and its CTA's factors.

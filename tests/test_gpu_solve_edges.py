@@ -4,7 +4,8 @@ solves of every field) against the oracle, and the same bits for every CTA size.
 A warp takes 32 degrees of one order, a CTA 1, 2 or 4 orders, a ring stage 4 rows.  The sizes put
 the last block of degrees at 1, 31, 8 and 1 degrees, orders that start inside a block, orders that
 are no multiple of a CTA's, every half-width KL, the fewest rows (N = 2 KL + 2), row counts that
-are no multiple of a stage, and the inner core's smallest and largest mesh.
+are no multiple of a stage, and the inner core's smallest and largest mesh.  Infinite and overflowing
+right-hand sides give the infinities and NaN of the divisions they stand for.
 
 Tolerance: FP64 on both sides in different orders; the toroidal velocity amplifies rounding most (the
 oracle's own change under last-bit perturbations of its initial state is 6e-11 of the largest
@@ -53,4 +54,61 @@ def test_steps_at_tile_edges(case):
                 assert np.abs(a - b).max() <= 1e-10 * max(np.abs(b).max(), 1e-300), f
         else:
             assert all(np.array_equal(a, b) for a, b in zip(first, got)), threads
+    o.close()
+
+
+def ieee_solve(ab, ipiv, kl, b):
+    """dgbtrs on the factors, without its tests for zero"""
+    n, b = b.size, b.copy()
+    for j in range(n):
+        p = ipiv[j] - 1
+        b[j], b[p] = b[p], b[j]
+        for i in range(1, min(kl, n - 1 - j) + 1):
+            b[j + i] -= ab[2 * kl + i, j] * b[j]
+    for j in range(n - 1, -1, -1):
+        b[j] = b[j] / ab[2 * kl, j]
+        for t in range(1, min(2 * kl, j) + 1):
+            b[j - t] -= b[j] * ab[2 * kl - t, j]
+    return b
+
+
+@pytest.mark.gpu
+def test_infinite_right_hand_sides():
+    import torch
+    cfg = capi.template_config(L=8, M=8, Mp=1, N=16, KL=3, timestep=1e-5, cod_bc=2)
+    g, o = pkg.Context(cfg), ol.Oracle(cfg)
+    l, _, _ = o.harmonics()
+    fields, lu = (capi.COD_C, capi.MAG_POL), (3, 5)
+    # rows of Re and Im of a harmonic: an infinity just inside the outer wall (it reaches the wall's row
+    # and its quotient), the largest magnitude there, an infinity in the middle, ordinary values
+    kinds = [(14, np.inf), (14, -np.inf), (14, np.finfo(float).max), (7, np.inf), (7, 1.0)]
+    b = np.ones((len(fields), cfg.N, g.H, 2))
+    b[:, [0, -1]] = 0.0
+    for nh in range(g.H):
+        for part in range(2):
+            row, v = kinds[(nh + 2 * part) % len(kinds)]
+            b[:, row, nh, part] = v
+    d = torch.tensor(b, device="cuda")
+    torch.cuda.synchronize()
+    g.operator_solve_device(list(fields), d.data_ptr())
+    g.synchronize()
+    x = d.cpu().numpy()
+    seen = 0
+    with np.errstate(all="ignore"):
+        for k, f in enumerate(fields):
+            for nh in range(g.H):
+                if f != capi.COD_C and l[nh] == 0:
+                    continue
+                ab, ipiv = o.operator_lu(lu[k], int(l[nh]))
+                for part in range(2):
+                    want, got = ieee_solve(ab, ipiv, cfg.KL, b[k, :, nh, part]), x[k, :, nh, part]
+                    assert np.array_equal(np.isnan(want), np.isnan(got)), (f, nh, part)
+                    inf = np.isinf(want)
+                    assert np.array_equal(inf, np.isinf(got)) and np.array_equal(want[inf], got[inf]), (f, nh, part)
+                    seen += inf.sum()
+                    fin = np.isfinite(want)
+                    if fin.all():
+                        assert np.abs(want - got).max() <= 1e-10 * np.abs(want).max(), (f, nh, part)
+    assert seen > 0
+    g.close()
     o.close()
