@@ -945,8 +945,19 @@ int dispatch_EG(int E, int G, F&& f) {
 
 bool lsd_fft_compiled(int E, int G) { return dispatch_EG(E, G, [](auto, auto) { return 0; }) == 0; }
 
+// The products' radices with the plan (E, G).  From E = 18 on a column pair no longer fits in a thread's
+// registers at G = 8 (E = 36: 3 KB of spills), so these plans' products run with the factor 2 back in the
+// row DFT; the grid transforms keep the plan.  us, as planned -> here, 33 shells, Boussinesq without
+// and anelastic with composition: M = 96 157, 339 -> 99, 222; M = 128 272, 583 -> 208, 391;
+// M = 192 1096, 2446 -> 456, 1106.
+struct ProdPlan { int E, G; };
+ProdPlan prod_plan(int E, int G) { return G == 8 && E >= 18 ? ProdPlan{E / 2, 16} : ProdPlan{E, G}; }
+
 // shared memory of the products kernel with the plan (E, G) for nfields staged rows
-size_t lsd_products_smem_for(int nfields, int E, int G) { return prod_smem(nfields, E, G); }
+size_t lsd_products_smem_for(int nfields, int E, int G) {
+  const ProdPlan p = prod_plan(E, G);
+  return prod_smem(nfields, p.E, p.G);
+}
 size_t lsd_products_smem_eg(const lsd_ctx* ctx, int E, int G) {
   const bool comp = ctx->cfg.comp_tstep != 0;
   int nf = comp ? 18 : 15;
@@ -1005,14 +1016,20 @@ namespace {
 template <int PS>
 int launch_products_set(lsd_ctx* ctx, const ProdConst& pc, const cplx* four_in, cplx* four_out) {
   FFTPlanDev pl = make_plan(ctx);
-  const size_t smem = prod_smem(PSet<PS>::in + PSet<PS>::deriv, ctx->fftE, ctx->fftG);
+  constexpr int NF = PSet<PS>::in + PSet<PS>::deriv;
+  const ProdPlan pp = prod_plan(ctx->fftE, ctx->fftG);
+  const size_t smem = prod_smem(NF, pp.E, pp.G);
   if (smem > 224 * 1024) return lsd_fail(ctx, LSD_EARG, "products: FFT rows do not fit in shared memory");
   dim3 grid(2 * ctx->HB, ctx->N);
-  int rc = dispatch_EG(ctx->fftE, ctx->fftG, [&](auto e, auto g) {
+  int rc = dispatch_EG(pp.E, pp.G, [&](auto e, auto g) {
     constexpr int E = decltype(e)::value, G = decltype(g)::value;
-    cudaFuncSetAttribute(k_products<E, G, PS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_products<E, G, PS><<<grid, ProdCfg<E, G, PS>::THREADS, smem, ctx->stream>>>(pl, ctx->N, pc, four_in, four_out);
-    return 0;
+    if constexpr ((G == 8 && E >= 18) || prod_smem(NF, E, G) > 224 * 1024) {
+      return -1;
+    } else {
+      cudaFuncSetAttribute(k_products<E, G, PS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      k_products<E, G, PS><<<grid, ProdCfg<E, G, PS>::THREADS, smem, ctx->stream>>>(pl, ctx->N, pc, four_in, four_out);
+      return 0;
+    }
   });
   if (rc) return lsd_fail(ctx, LSD_EARG, "FFT length not supported");
   ctx->launches++;
