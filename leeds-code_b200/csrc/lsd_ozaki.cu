@@ -838,23 +838,23 @@ constexpr int OZ_MAXG_SYNTH = OZ_MAXG, OZ_MAXG_ANAL = 4;  // groups per launch
 // the digit / exponent buffer of each type's chain
 int oz_buf(int type) { return type == OZ_VEC || type == OZ_ST ? 0 : type == OZ_P || type == OZ_Q ? 1 : 2; }
 
-// f(integral_constant S) for the runtime slice count S
-template <int TYPE, class F>
-void oz_slices_dispatch(int S, F&& f) {
+// f(integral_constant S) for the runtime slice count S; false: no kernel for that count
+template <class F>
+bool oz_slices_dispatch(int S, F&& f) {
   switch (S) {
-    case 2: f(std::integral_constant<int, 2>()); break;
-    case 3: f(std::integral_constant<int, 3>()); break;
-    case 4: f(std::integral_constant<int, 4>()); break;
-    case 5: f(std::integral_constant<int, 5>()); break;
-    case 6: f(std::integral_constant<int, 6>()); break;
-    case 7: f(std::integral_constant<int, 7>()); break;
-    case 8: f(std::integral_constant<int, 8>()); break;
-    default: break;
+    case 2: f(std::integral_constant<int, 2>()); return true;
+    case 3: f(std::integral_constant<int, 3>()); return true;
+    case 4: f(std::integral_constant<int, 4>()); return true;
+    case 5: f(std::integral_constant<int, 5>()); return true;
+    case 6: f(std::integral_constant<int, 6>()); return true;
+    case 7: f(std::integral_constant<int, 7>()); return true;
+    case 8: f(std::integral_constant<int, 8>()); return true;
+    default: return false;
   }
 }
 template <int TYPE>
 void oz_set_smem(int S, size_t smem) {
-  oz_slices_dispatch<TYPE>(S, [&](auto sc) {
+  oz_slices_dispatch(S, [&](auto sc) {
     cudaFuncSetAttribute(k_oz_gemm<TYPE, decltype(sc)::value>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   });
 }
@@ -1094,12 +1094,13 @@ int oz_run(lsd_ctx* ctx, const OzLaunchGroup* gs, int ng, cudaStream_t stream) {
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->dev);
   const int ntile = ctx->NM * 2 * nzb;
-  oz_slices_dispatch<TYPE>(o->S, [&](auto sc) {
+  const bool known = oz_slices_dispatch(o->S, [&](auto sc) {
     constexpr int S = decltype(sc)::value;
     cudaFuncSetAttribute(k_oz_prep<TYPE, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm);
     k_oz_prep<TYPE, S><<<pg, 256, psm, stream>>>(pa, srow);
     k_oz_gemm<TYPE, S><<<std::min(ntile, o->ctas * nsm), OZ_THREADS, o->smem, stream>>>(ga, nzb);
   });
+  if (!known) return lsd_fail(ctx, LSD_EARG, "tensor-core contraction: no kernel for this number of slices");
   ctx->launches += 2;
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return lsd_fail(ctx, LSD_ECUDA, std::string("tensor-core contraction: ") + cudaGetErrorString(e));
