@@ -930,8 +930,21 @@ int lsd_ozaki_setup(lsd_ctx* ctx) {
   o->S = S;
   oz_route(ctx, o);
   const int NM = ctx->NM, Th2 = ctx->Th2, N = ctx->N;
-  for (int c = 0; c < NM; ++c)
-    if (ctx->mlen[c] > 512) return lsd_fail(ctx, LSD_EARG, "tensor-core path: more than 512 harmonics per m");
+  // The limits of the slices hold for a context of any route, so which sizes are accepted does not depend
+  // on the lines of oz_route.
+  int mx = 1;
+  for (int c = 0; c < NM; ++c) mx = std::max(mx, ctx->mlen[c]);
+  if (mx > 512) return lsd_fail(ctx, LSD_EARG, "tensor-core path: more than 512 harmonics per m");
+  o->srow[0] = mx | 1;
+  o->srow[1] = (2 * Th2) | 1;
+  if (oz_prep_smem<OZ_ST>(o->srow[1]) > 200 * 1024 || oz_prep_smem<OZ_VEC>(o->srow[0]) > 200 * 1024)
+    return lsd_fail(ctx, LSD_EARG, "tensor-core path: pre-pass rows do not fit in shared memory");
+  // ring stages: as many (2..4) as keep two CTAs per SM (<= 78 KiB of stages each)
+  lsd_ozaki_default_tiles(S, &o->nst, &o->ctas);
+  o->smem = (size_t)o->nst * oz_stage_bytes(S);
+  CUDA_TRY(cudaMalloc(&o->d_err, sizeof(int)));
+  CUDA_TRY(cudaMemsetAsync(o->d_err, 0, sizeof(int), ctx->stream));
+  if (!o->synth && !o->anal) return LSD_OK;  // no tables, no digit buffers
   std::vector<std::vector<int>> Kcp((size_t)NM * 2);  // harmonics per (counter, parity)
   for (int c = 0; c < NM; ++c)
     for (int k = 0; k < ctx->mlen[c]; ++k) {
@@ -944,6 +957,7 @@ int lsd_ozaki_setup(lsd_ctx* ctx) {
   int fofs = 0;
   for (int type = 0; type < OZ_NTYPE; ++type) {
     const bool anal = type >= OZ_ST;
+    if (!(anal ? o->anal : o->synth)) continue;  // that direction runs on the FP64 instruction
     const int per = (type == OZ_P || type == OZ_Q) ? 2 : 4;
     const int maxg = anal ? OZ_MAXG_ANAL : OZ_MAXG_SYNTH;
     o->nzb_max[type] = ceil_div(maxg * per * N, 128);
@@ -1006,20 +1020,6 @@ int lsd_ozaki_setup(lsd_ctx* ctx) {
     for (int d = 0; d < S; ++d) total += (double)bound(d) * std::ldexp(1.0, 8 * (S - 1 - d));
     o->wide[type] = total < std::ldexp(1.0, 62) ? 1 : 0;
   }
-  // ring stages: as many (2..4) as keep two CTAs per SM (<= 78 KiB of stages each)
-  lsd_ozaki_default_tiles(S, &o->nst, &o->ctas);
-  o->smem = (size_t)o->nst * oz_stage_bytes(S);
-  {
-    int mx = 1;
-    for (int c = 0; c < NM; ++c) mx = std::max(mx, ctx->mlen[c]);
-    o->srow[0] = mx | 1;
-    o->srow[1] = (2 * Th2) | 1;
-    if (oz_prep_smem<OZ_ST>(o->srow[1]) > 200 * 1024 || oz_prep_smem<OZ_VEC>(o->srow[0]) > 200 * 1024)
-      return lsd_fail(ctx, LSD_EARG, "tensor-core path: pre-pass rows do not fit in shared memory");
-  }
-  CUDA_TRY(cudaMalloc(&o->d_err, sizeof(int)));
-  CUDA_TRY(cudaMemsetAsync(o->d_err, 0, sizeof(int), ctx->stream));
-  if (!lsd_ozaki_use_synth(ctx) && !lsd_ozaki_use_anal(ctx)) return LSD_OK;  // no tables, no digit buffers
   if (kidx.empty()) kidx.push_back(0);
   if (nhl.empty()) nhl.push_back(0);
   CUDA_TRY(cudaMalloc(&o->d_probs, sizeof(OzProb) * probs.size()));
@@ -1049,9 +1049,10 @@ int lsd_ozaki_setup(lsd_ctx* ctx) {
   const int t2[OZ_NTYPE] = {LSD_LEG_LLSIN1MP, LSD_LEG_P, LSD_LEG_SIN1MP, LSD_LEG_GWLLSIN1MP, LSD_LEG_GWP};
   for (int i = 0; i < OZ_NTYPE; ++i) { ta.tab1[i] = t1[i]; ta.tab2[i] = t2[i]; }
   const dim3 g(NM, 2);
-  for (int type = OZ_VEC; type <= OZ_GRAD; ++type) k_oz_tab_synth<<<g, 128, 0, ctx->stream>>>(ta, type);
-  for (int type = OZ_ST; type <= OZ_Q; ++type) k_oz_tab_anal<<<g, 64, 0, ctx->stream>>>(ta, type);
-  ctx->launches += 5;
+  if (o->synth)
+    for (int type = OZ_VEC; type <= OZ_GRAD; ++type, ctx->launches++) k_oz_tab_synth<<<g, 128, 0, ctx->stream>>>(ta, type);
+  if (o->anal)
+    for (int type = OZ_ST; type <= OZ_Q; ++type, ctx->launches++) k_oz_tab_anal<<<g, 64, 0, ctx->stream>>>(ta, type);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   oz_set_smem<OZ_VEC>(o->S, o->smem); oz_set_smem<OZ_P>(o->S, o->smem); oz_set_smem<OZ_GRAD>(o->S, o->smem);

@@ -43,12 +43,18 @@ def route(g):
     (208, 32, 1, 7, (True, True)), (204, 128, 1, 7, (True, True)),
     # and 0.4 .. 1.02 times at these
     (128, 16, 1, 6, (False, False)), (192, 192, 1, 6, (False, False)), (192, 32, 6, 6, (False, False)),
-    (256, 256, 1, 7, (False, False)), (192, 96, 1, 7, (False, False)), (153, 48, 1, 7, (True, False)), (256, 32, 8, 7, (False, False)), (64, 16, 4, 7, (False, False)),
+    (256, 256, 1, 7, (False, False)), (192, 96, 1, 7, (False, False)), (256, 32, 8, 7, (False, False)),
+    (192, 64, 1, 7, (False, True)), (153, 48, 1, 7, (True, False)), (64, 16, 4, 7, (False, False)),
     (64, 16, 4, 5, (True, True)), (64, 16, 4, 8, (True, True))])
 def test_faster_side_of_the_dispatch(L, M, Mp, S, int8):
-    g = pkg.Context(capi.template_config(L=L, M=M, Mp=Mp, N=6, KL=2, timestep=1e-5, precision=capi.PREC_OZAKI,
-                                         ozaki_slices=S))
+    """also: lsd_create makes the three (synthesis) and two (analysis) digit tables of the directions
+    that read them"""
+    kw = dict(L=L, M=M, Mp=Mp, N=6, KL=2, timestep=1e-5)
+    f = pkg.Context(capi.template_config(**kw))
+    g = pkg.Context(capi.template_config(precision=capi.PREC_OZAKI, ozaki_slices=S, **kw))
+    assert g.kernel_launches() - f.kernel_launches() == 3 * int8[0] + 2 * int8[1]
     assert route(g) == int8
+    f.close()
     g.close()
 
 
