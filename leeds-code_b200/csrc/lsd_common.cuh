@@ -254,6 +254,7 @@ int lsd_ozaki_set_tiles(lsd_ctx* ctx, int nst, int ctas);
 // ---- autotuner (lsd_tune.cu) ----
 bool lsd_fft_compiled(int E, int G);
 size_t lsd_products_smem_for(int nfields, int E, int G);
+bool lsd_products_own_plan(int E, int G);  // the products run with this plan, not with the default's radices
 int lsd_autotune(lsd_ctx* ctx);
 
 // small helpers

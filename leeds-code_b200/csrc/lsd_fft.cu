@@ -953,6 +953,8 @@ bool lsd_fft_compiled(int E, int G) { return dispatch_EG(E, G, [](auto, auto) { 
 struct ProdPlan { int E, G; };
 ProdPlan prod_plan(int E, int G) { return G == 8 && E >= 18 ? ProdPlan{E / 2, 16} : ProdPlan{E, G}; }
 
+bool lsd_products_own_plan(int E, int G) { return prod_plan(E, G).G == G; }
+
 // shared memory of the products kernel with the plan (E, G) for nfields staged rows
 size_t lsd_products_smem_for(int nfields, int E, int G) {
   const ProdPlan p = prod_plan(E, G);

@@ -154,6 +154,10 @@ int lsd_autotune(lsd_ctx* ctx) {
   {
     std::vector<double> ms(sp.nfft, 0.0);
     for (int i = 0; i < sp.nfft; ++i) {
+      if (!lsd_products_own_plan(sp.fft_E[i], sp.fft_G[i])) {  // an evaluation is the default plan's
+        ms[i] = 1e30;
+        continue;
+      }
       ctx->fftE = sp.fft_E[i];
       ctx->fftG = sp.fft_G[i];
       int rc = time_ms(ctx, [&]() { return lsd_eval(ctx); }, reps, &ms[i]);
@@ -166,8 +170,9 @@ int lsd_autotune(lsd_ctx* ctx) {
     ctx->fftE = ch.E;
     ctx->fftG = ch.G;
   }
-  // tensor-core GEMM tiles: one evaluation each
-  if (ctx->oz && sp.ngemm > 0) {
+  // tensor-core GEMM tiles: one evaluation each, where a direction runs on the slices (else the
+  // defaults stay and ms_gemm is 0)
+  if ((lsd_ozaki_use_synth(ctx) || lsd_ozaki_use_anal(ctx)) && sp.ngemm > 0) {
     std::vector<double> ms(sp.ngemm, 0.0);
     for (int i = 0; i < sp.ngemm; ++i) {
       int rc = lsd_ozaki_set_tiles(ctx, sp.gemm_stages[i], sp.gemm_ctas[i]);

@@ -4,9 +4,10 @@ CPU: the candidate lists of several configurations (every phi-FFT plan multiplie
 P2 = 3M/2 and is compiled, the default plan comes first, the tensor-core GEMM's tiles
 respect the shared-memory limit of their CTAs per SM) and the selection rule on made-up
 timings.
-GPU: a tuned context reports parameters from its candidate lists; the solve mapping (CTA
-size) leaves every bit of a run unchanged; another FFT plan changes coefficients only at
-the rounding level (1e-12); a tuned context steps like an untuned one.
+GPU: a tuned context reports parameters from its candidate lists and times no kernel that
+it does not launch; the solve mapping (CTA size) leaves every bit of a run unchanged; another
+FFT plan changes coefficients only at the rounding level (1e-12); a tuned context steps like
+an untuned one.
 """
 import importlib
 
@@ -120,3 +121,17 @@ def test_other_fft_plan(parity_report):
             worst = max(worst, d)
         parity_report("FFT plan (%d, %d) vs default, coefficients after 3 steps" % (E, G), worst, 1e-12)
         assert worst <= 1e-12, (E, G, worst)
+
+
+@pytest.mark.gpu
+def test_only_kernels_that_run_are_timed():
+    """seven slices at this size run on the FP64 instruction: the tiles of the slices' GEMM stay at their
+    defaults, untimed; the products of the plan (18, 8) run as the default plan's"""
+    kw = dict(L=97, M=96, N=17, precision=capi.PREC_OZAKI, ozaki_slices=7)
+    plain, tuned = pkg.Context(syn.config_parity(**kw)), pkg.Context(syn.config_parity(autotune=1, **kw))
+    a, b = plain.tuning(), tuned.tuning()
+    assert b["tuned"] == 1 and b["ms_gemm"] == 0 and b["ms_fft"] > 0 and b["ms_solve"] > 0
+    assert (a["gemm_stages"], a["gemm_ctas_per_sm"]) == (b["gemm_stages"], b["gemm_ctas_per_sm"])
+    assert (18, 8) in lsd.tune_candidates(tuned.cfg)["fft"] and (b["fft_E"], b["fft_G"]) == (9, 16)
+    plain.close()
+    tuned.close()
