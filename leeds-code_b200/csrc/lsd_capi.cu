@@ -39,7 +39,7 @@ void free_ctx(lsd_ctx* ctx) {
     cudaEventDestroy(x.fork);
   }
   lsd_ozaki_free(ctx);
-  void* ptrs[] = {ctx->d_l, ctx->d_m, ctx->d_s, ctx->d_mc, ctx->d_mstart, ctx->d_mlen, ctx->d_thm, ctx->d_bin2c, ctx->d_lm2nh,
+  void* ptrs[] = {ctx->d_l, ctx->d_m, ctx->d_mstart, ctx->d_mlen, ctx->d_thm, ctx->d_bin2c, ctx->d_lm2nh,
                   ctx->d_leg, ctx->d_gp, ctx->d_gw, ctx->d_sn, ctx->d_sn1, ctx->d_tw2, ctx->d_twh, ctx->d_r,
                   ctx->d_dr, ctx->d_r1dr, ctx->d_radlap, ctx->d_intr2dr, ctx->d_lu, ctx->d_y, ctx->d_lf, ctx->d_uf, ctx->d_yf,
                   ctx->d_ipiv, ctx->d_info, ctx->d_gf, ctx->d_invg, ctx->d_state, ctx->d_nl,
@@ -91,7 +91,7 @@ int h2d(lsd_ctx* ctx, void* d, const void* h, size_t bytes) {
 
 // harmonic layout: _loop_setlm (parallel.h_template:54-80), _loop_sumth (:85-100)
 void build_layout(lsd_ctx* c) {
-  c->hl.assign(c->H, 0); c->hm.assign(c->H, 0); c->hs.assign(c->H, 0); c->mcount.assign(c->H, 0);
+  c->hl.assign(c->H, 0); c->hm.assign(c->H, 0); c->hs.assign(c->H, 0);
   int nh = -1;
   for (int j = 1; j <= c->Hc; ++j)
     for (int i = 1; i <= c->Hr; ++i) {
@@ -108,7 +108,6 @@ void build_layout(lsd_ctx* c) {
     int m__ = m_;
     m_ = c->hm[nh];
     if (m_ != m__) { ++m; c->thm[m] = m_ / c->Mp; c->mstart[m] = nh; }
-    c->mcount[nh] = m;
     c->mlen[m]++;
   }
 }
@@ -584,8 +583,6 @@ int lsd_create(const lsd_config* cfg, lsd_ctx** out) {
   for (int nh = 0; nh < H; ++nh) lm2nh[(size_t)(ctx->hm[nh] / ctx->Mp) * L + ctx->hl[nh]] = nh;
   TRY(dalloc(ctx, &ctx->d_l, H)); TRY(upload(ctx, ctx->d_l, ctx->hl));
   TRY(dalloc(ctx, &ctx->d_m, H)); TRY(upload(ctx, ctx->d_m, ctx->hm));
-  TRY(dalloc(ctx, &ctx->d_s, H)); TRY(upload(ctx, ctx->d_s, ctx->hs));
-  TRY(dalloc(ctx, &ctx->d_mc, H)); TRY(upload(ctx, ctx->d_mc, ctx->mcount));
   TRY(dalloc(ctx, &ctx->d_mstart, NM)); TRY(upload(ctx, ctx->d_mstart, ctx->mstart));
   TRY(dalloc(ctx, &ctx->d_mlen, NM)); TRY(upload(ctx, ctx->d_mlen, ctx->mlen));
   TRY(dalloc(ctx, &ctx->d_thm, NM)); TRY(upload(ctx, ctx->d_thm, ctx->thm));

@@ -108,9 +108,9 @@ struct lsd_ctx {
   cudaEvent_t ev_staged[2] = {nullptr, nullptr}, ev_committed[2] = {nullptr, nullptr};
 
   // host layout
-  std::vector<int> hl, hm, hs, thm, mcount, mstart, mlen;
+  std::vector<int> hl, hm, hs, thm, mstart, mlen;
   // device layout
-  int *d_l = nullptr, *d_m = nullptr, *d_s = nullptr, *d_mc = nullptr;
+  int *d_l = nullptr, *d_m = nullptr;
   int *d_mstart = nullptr, *d_mlen = nullptr, *d_thm = nullptr, *d_lm2nh = nullptr, *d_bin2c = nullptr;
   int nh_l1m0 = -1, nh_l1m1 = -1;  // toroidal modes of vel_angmomclr
   // device Legendre tables, each [H][Th2] (== Fortran (Th2, H))

@@ -343,6 +343,7 @@ int lsd_launch_synth(lsd_ctx* ctx, const SynthGroup* groups, int ngroups) {
 
 int lsd_launch_anal(lsd_ctx* ctx, const AnalGroup* groups, int ngroups) {
   if (lsd_ozaki_use_anal(ctx)) return lsd_ozaki_launch_anal(ctx, groups, ngroups);
+  // k_leg has no such limit; longer columns (L > 512) are outside what is tested
   if (ceil_div(ctx->Hr, 32) * 32 > 1024) return lsd_fail(ctx, LSD_EARG, "analysis: folded column longer than 1024 harmonics");
   LegBuilder b;
   bool ok = true;

@@ -226,7 +226,7 @@ struct StepArgs {
   int comp;
   double* cpart;  // corrector: the per-warp sums [8][nwarp] that k_cgce_sums adds up
   int nwarp;      // (blocks of 32 degrees) x orders
-  int NL;       // rows per operator in lus / ipivs (N + Nic - 1)
+  int NL;       // rows per family of lf and uf (N + Nic - 1)
   int Nic;      // inner-core points (> 1: conducting, the field families are coupled)
   cplx* icstate;       // [2][Nic][H] mag_icTor, mag_icPol
   cplx* icsv;          // [2][Nic][H] their saved nonlinear terms

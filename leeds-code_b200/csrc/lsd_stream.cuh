@@ -3,9 +3,9 @@
 // A warp owns 32 consecutive degrees l of one order m (lane = degree) and walks the radial rows of
 // their columns; a CTA takes the same 32 degrees of T / 32 orders, so its warps share the factors,
 // which depend on l alone.  The rows of a pass -- the lane's own column values and the CTA's
-// factor rows -- arrive by 16-byte asynchronous copies in a ring of SV_ST stages of SV_B rows, 8 to
-// 16 rows ahead of the arithmetic; rows outside the system arrive as zeros, so that every step of
-// a pass does the same work and only its stores are guarded.
+// factor rows -- arrive by 16-byte asynchronous copies in a ring of SvRing::ST stages of SV_B rows, 12
+// rows ahead of the arithmetic (8 for KL > 3); rows outside the system arrive as zeros, so that
+// every step of a pass does the same work and only its stores are guarded.
 //
 // Factors in the solve layouts: per (family, block of 32 degrees) the rows -SV_PAD .. NL + SV_PAD - 1
 // (zeros outside the system) of
@@ -18,13 +18,13 @@
 // way) and, with many columns, the instructions of a row.  So no load stands in the chain (a
 // row loaded when it is needed costs 0.7 us per batch of rows) and no division (114 cycles): x / d is
 // formed from the stored reciprocal with one correction step (Markstein, IBM J. Res. Dev. 34, 111
-// (1990): q = x r, then q + (x - q d) r).  q is off by at most 2^-52 of itself and r by 2^-53 of itself,
-// so the sum before its rounding is off by 2^-105: the rounded quotient, but for quotients that close to a
-// tie, as long as r is a normal number (the factorisation multiplies by the same reciprocals) and
-// |x| is above 2^-968, where x - q d is exact.  Sharing the factors between four orders takes their traffic from 84 to 21 bytes
-// per column row and pass.  All passes of a column run through one copy of the code (a loop
-// over pass descriptors): with a copy per pass the short columns of a small run waited for
-// instruction fetches half of their time.
+// (1990): q = x r, then q + (x - q d) r).  q is off by at most 2^-52 of itself and r by 2^-53, so
+// the sum before its rounding is off by 2^-105: the rounded quotient, but for quotients that
+// close to a tie, as long as r is a normal number (the factorisation multiplies by the same
+// reciprocals) and |x| is above 2^-968, where x - q d is exact.  Sharing the factors between four
+// orders takes their traffic from 84 to 21 bytes per column row and pass.  All passes of a column
+// run through one copy of the code (a loop over pass descriptors): with a copy per pass the
+// short columns of a small run waited for instruction fetches half of their time.
 // Five fields of a step (8256 harmonics, N = 129, KL = 3): predictor 0.150 ms, corrector 0.163 ms; one
 // thread per harmonic with batches of eight rows loaded when needed 0.367 and 0.355 ms.  At L = 16,
 // N = 17: 26 and 28 us (37 and 40).  Five fields at N = 257, KL = 4, 32896 harmonics (operator
