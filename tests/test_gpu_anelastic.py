@@ -13,7 +13,9 @@ Oracle pins (CPU):
     to the Boussinesq ones bit for bit.
 Parity (GPU, relative to the largest magnitude of the compared array):
   unit transforms 1e-12; one evaluation, predictor and corrector 1e-11 (FP64), 5e-11
-  (tensor cores, S = 7); 100 steps: energies 1e-9, coefficients 1e-10.
+  (S = 7, which is FP64 at this size, and S = 8, tensor cores), 7e-10 (S = 5, tensor cores: 4
+  times the measured 1.7e-10; the energies 5e-8, 4 times 1.3e-8); 100 steps: energies 1e-9,
+  coefficients 1e-10.
 """
 import importlib
 import os
@@ -126,8 +128,9 @@ def test_anelastic_unit_transforms():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("prec,S,tol", [(capi.PREC_FP64, 0, 1e-11), (capi.PREC_OZAKI, 7, 5e-11)])
-def test_anelastic_evaluation_and_step(prec, S, tol):
+@pytest.mark.parametrize("prec,S,tol,tol_e", [(capi.PREC_FP64, 0, 1e-11, 1e-10), (capi.PREC_OZAKI, 7, 5e-11, 1e-10),
+                                              (capi.PREC_OZAKI, 8, 5e-11, 1e-10), (capi.PREC_OZAKI, 5, 7e-10, 5e-8)])
+def test_anelastic_evaluation_and_step(prec, S, tol, tol_e):
     cfg = anel_cfg()
     g = pkg.Context(anel_cfg(precision=prec, ozaki_slices=S))
     o = ol.Oracle(cfg)
@@ -155,7 +158,7 @@ def test_anelastic_evaluation_and_step(prec, S, tol):
         assert relerr(a[1], b[1]) < tol, ("corr", f)
     ea, eb = g.energies(), o.energies()
     for k in ("KE", "ME", "KE_dis", "ME_dis", "topflx", "botflx", "KE_ax", "ME_ax"):
-        assert abs(ea[k] - eb[k]) <= 1e-10 * abs(eb[k]), (k, ea[k], eb[k])
+        assert abs(ea[k] - eb[k]) <= tol_e * abs(eb[k]), (k, ea[k], eb[k])
     g.close()
     o.close()
 

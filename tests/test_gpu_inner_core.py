@@ -10,8 +10,8 @@ io_ic_extend (a r^3 + b r^2) and rot_omega = 1.5.
 * The same with the CFL / corrector-controlled dt (d_timestep = -5e-5), 20 steps: the dt
   sequence (1e-9) and rot_omega.
 * The case 2 resolution of the reference's INFO file (L = 64, M = 16, Mp = 4, N = 64,
-  Nic = 16), tensor-core Legendre transforms, 3 steps against the FP64 oracle: fields and
-  rotation to 1e-9.
+  Nic = 16), 3 steps against the FP64 oracle with the default slice count (FP64 at this size) and
+  with 5 and 8 slices (tensor-core Legendre transforms): fields and rotation to 1e-9.
 * Free decay of the whole conducting sphere on the device (Ra = 0, field 1e-7): the decay
   rates of the l = 1 poloidal and toroidal modes equal the oracle's to 1e-9 and 2 k^2
   (poloidal) to 1e-6.
@@ -100,8 +100,10 @@ def test_inner_core_variable_dt():
 
 
 @pytest.mark.gpu
-def test_inner_core_case2_resolution_tensor_cores():
-    cfg = syn.config_inner_core(L=64, M=16, Mp=4, N=64, Nic=16, KL=4, precision=capi.PREC_OZAKI, timestep=2e-5)
+@pytest.mark.parametrize("S", [0, 5, 8])
+def test_inner_core_case2_resolution_tensor_cores(S):
+    cfg = syn.config_inner_core(L=64, M=16, Mp=4, N=64, Nic=16, KL=4, precision=capi.PREC_OZAKI, ozaki_slices=S,
+                                timestep=2e-5)
     ocfg = syn.config_inner_core(L=64, M=16, Mp=4, N=64, Nic=16, KL=4, timestep=2e-5)
     g, o = pkg.Context(cfg), ol.Oracle(ocfg)
     st, om = start(cfg, o, seed=41, omega=-13.3)
