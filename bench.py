@@ -31,9 +31,11 @@ cpu_baseline: the CPU oracle (C++ restatement of the reference path, OpenMP over
 Other scope configurations (one JSON line each, same keys):
   --workload sht256    the SHT round trip at lmax = mmax = 255 (L = M = 256, Th = 384,
          Ph = 768), 64 shells x 8 fields, device-resident synthesis + analysis
-         (lsd_sht_*_device); value = SHT TF/s (Legendre + FFT algorithmic flops) of the
-         tensor-core contraction at 7 slices, every variant (FP64, 8/7/5/4 slices) listed
-         with its time and its error against the FP64 variant per field.
+         (lsd_sht_*_device); value = SHT TF/s (Legendre + FFT algorithmic flops) of a
+         context of 7 slices, every variant (FP64, 8/7/5/4 slices) listed with the contraction
+         that each direction ran (int8 slices, or the FP64 tensor instruction where the
+         library takes that: 7 slices at this size), its time and its error against the FP64
+         variant per field.
   --workload solve257  the batched banded solves at N = 257, KL = 4, L = M = 256: every
          (l, m) right-hand side of five fields (codensity, toroidal velocity, the field's
          toroidal / poloidal scalars, the poloidal velocity's fourth-order composite) on the
@@ -236,7 +238,7 @@ def energy_check(args, local_rank, nsteps):
 # DRAM traffic per launch of the dominant kernel from an ncu capture of this benchmark
 # (dram__bytes_read.sum + dram__bytes_write.sum); see profiles/ for the command.
 NCU_TRAFFIC = {
-    "fft_products": {"kernel": "k_products<12,16>", "bytes": 760.93e6 + 331.13e6,
+    "fft_products": {"kernel": "k_products<12,16>", "bytes": 761.50e6 + 331.17e6,
                      "profile": "profiles/k_products_dynamo128.md"},
 }
 
@@ -328,6 +330,18 @@ SHT256_VARIANTS = [("fp64", 0), ("ozaki", 8), ("ozaki", 7), ("ozaki", 5), ("ozak
 SHT256_HEADLINE = ("ozaki", 7)
 
 
+def contractions(ctx, d_spec, d_phys, d_back):
+    """which contraction each direction runs, from the launches of a one-field transform: the
+    slices take two (slicing pass, GEMM), the FP64 contraction one, the phi FFT one more"""
+    n = [ctx.kernel_launches()]
+    ctx.sht_synth_device(1, d_spec, d_phys)
+    n.append(ctx.kernel_launches())
+    ctx.sht_analys_device(1, d_phys, d_back)
+    n.append(ctx.kernel_launches())
+    name = {2: "fp64", 3: "int8 slices"}
+    return {"synthesis": name[n[1] - n[0]], "analysis": name[n[2] - n[1]]}
+
+
 def run_sht256(args, rank, world, local_rank, dist):
     """config[1]: SHT round trips of 64 shells x 8 fields at L = M = 256"""
     import torch
@@ -356,6 +370,7 @@ def run_sht256(args, rank, world, local_rank, dist):
         def round_trip():
             ctx.sht_synth_device(nf, d_spec.data_ptr(), d_phys.data_ptr())
             ctx.sht_analys_device(nf, d_phys.data_ptr(), d_back.data_ptr())
+        ran = contractions(ctx, d_spec.data_ptr(), d_phys.data_ptr(), d_back.data_ptr())
         for _ in range(args.warmup):
             round_trip()
         ctx.synchronize()
@@ -393,7 +408,8 @@ def run_sht256(args, rank, world, local_rank, dist):
         e2e_ms = stop(cur) / ne
         if dist:
             e2e_ms = max_over_ranks(dist, e2e_ms, "cuda:%d" % local_rank)
-        out[(prec, S)] = {"ms": ms, "e2e_ms": e2e_ms, "launches": launches, "err_synth_vs_fp64": max(e_syn),
+        out[(prec, S)] = {"ms": ms, "contractions": ran, "e2e_ms": e2e_ms, "launches": launches,
+                          "err_synth_vs_fp64": max(e_syn),
                           "err_round_trip_vs_fp64": max(e_rt), "err_round_trip_vs_input": max(e_in),
                           "sizes": ctx.sizes}
         torch.cuda.synchronize()
@@ -415,7 +431,7 @@ def run_sht256(args, rank, world, local_rank, dist):
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f64",
         "data": "synthetic (seeded N(0,1) l^-1 coefficients)",
         "config": {"workload": "SHT round trip lmax=mmax=255 (L=M=256), Th=384, Ph=768, 64 shells x 8 fields",
-                   "precision": "ozaki", "ozaki_slices": SHT256_HEADLINE[1],
+                   "precision": "ozaki", "ozaki_slices": SHT256_HEADLINE[1], "contractions": h["contractions"],
                    "l2": "per-trip working set ~3 GB >> 126 MB L2 (no flush)"},
         "e2e": {"value": world * (leg + fft) / (h["e2e_ms"] * 1e-3) / 1e12, "unit": "TF/s",
                 "h2d_bytes_per_step": nf * N * H * 16, "d2h_bytes_per_step": nf * N * H * 16},
@@ -425,7 +441,8 @@ def run_sht256(args, rank, world, local_rank, dist):
         "roofline_note": "whole round trip: algorithmic bytes (spectra in/out, the physical grid written "
                          "and read) over its device time; peak %s" % src,
         "variants": {("%s_S%d" % k if k[0] == "ozaki" else "fp64"): {
-            "ms": v["ms"], "tflops": world * (leg + fft) / (v["ms"] * 1e-3) / 1e12,
+            "contractions": v["contractions"], "ms": v["ms"],
+            "tflops": world * (leg + fft) / (v["ms"] * 1e-3) / 1e12,
             "err_synth_vs_fp64": v["err_synth_vs_fp64"], "err_round_trip_vs_fp64": v["err_round_trip_vs_fp64"],
             "err_round_trip_vs_input": v["err_round_trip_vs_input"]} for k, v in out.items()},
     }
@@ -810,7 +827,7 @@ def run_ours(args, rank, world, local_rank, dist):
         ctx.synchronize()
         res["e2e_s"] = max_over_ranks(dist, (time.perf_counter() - t0) / ne, "cuda:%d" % local_rank)
         res["h2d"] = 5 * ctx.N * ctx.H * 16
-        res["d2h"] = (48 + 2) * ctx.N * 8 + 3 * 16
+        res["d2h"] = ((69 + 2 * cfg.KL) * ctx.N + 6) * 8  # the norms and what the radial sums need
         ph, rf = phase_roofline(ctx, peaks, src)
         res["phases_ms"] = ph
         res["roofline"] = rf

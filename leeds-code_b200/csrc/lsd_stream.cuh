@@ -27,8 +27,8 @@
 // short columns of a small run waited for instruction fetches half of their time.
 // Five fields of a step (8256 harmonics, N = 129, KL = 3): predictor 0.150 ms, corrector 0.163 ms; one
 // thread per harmonic with batches of eight rows loaded when needed 0.367 and 0.355 ms.  At L = 16,
-// N = 17: 26 and 28 us (37 and 40).  Five fields at N = 257, KL = 4, 32896 harmonics (operator
-// solves) 0.94 ms (1.20).
+// N = 17: 25 and 30 us (37 and 40).  Five fields at N = 257, KL = 4, 32896 harmonics (operator
+// solves) 0.75 ms (1.14).
 #pragma once
 #include "lsd_common.cuh"
 
