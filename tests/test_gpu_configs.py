@@ -13,7 +13,7 @@ counts (S balanced base-256 int8 digits, 8S - 2 bits of the FP64 mantissa, round
 Tolerances, relative to the largest magnitude of the compared field:
   FP64            synthesis, analysis, round trip vs the oracle's: 1e-12
   tensor, S = 8   1e-13
-  tensor, S = 7   5e-12
+  tensor, S = 7   5e-12   (runs as FP64 at this size)
   tensor, S = 5   2e-8    (38 bits)
   tensor, S = 4   1e-6    (30 bits, about FP32)
 config[2]: batched banded solves at N = 257, KL = 4.
