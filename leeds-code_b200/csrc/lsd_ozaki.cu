@@ -876,22 +876,22 @@ void oz_set_smem(int S, size_t smem) {
 // order; the FP64 contraction pays for theta rows padded to tiles of 48 (synthesis, a factor pad) and for
 // the 8-byte table copies of an odd half grid (15 %, odd).  FP64 / int8 measured at 62 shapes (L 64 .. 264,
 // M 12 .. 256, Mp 1 .. 12, N 20 .. 99; the geometric mean in brackets):
-//   synthesis  S = 6: K pad odd <= 122 0.40 .. 1.06 (0.67), up to 152 0.86 .. 1.18 (0.98), above 0.76 .. 1.50 (1.11)
+//   synthesis  S = 6: K pad odd <= 130 0.40 .. 1.06 (0.72), up to 162 0.88 .. 1.18 (1.01), above 0.76 .. 1.50 (1.11)
 //              S = 7:           <= 175 0.39 .. 0.99 (0.72), up to 219 0.70 .. 1.25 (0.93), above 0.69 .. 1.26 (0.99)
 //   analysis   S = 6: K odd     <= 124 0.47 .. 1.06 (0.76), up to 155 0.61 .. 1.15 (0.99), above 0.70 .. 1.44 (1.06)
 //              S = 7:           <= 160 0.46 .. 1.02 (0.77), up to 200 0.65 .. 1.08 (0.90), above 0.73 .. 1.25 (1.00)
 // Beyond the bounds int8 also keeps shapes of few columns (M = 16, N = 33), where FP64 would win.
 // Up to five slices int8 stays at all sizes, though FP64 is faster at most of them: it would move the
 // outputs of such a run by the slices' own rounding (two steps of an anelastic member at five slices by
-// 1.9e-10 of the largest coefficient).  Eight slices stay for
-// their precision, 62 bits of each row or column maximum and exact digit sums: sums of 32 products that
-// rise to 5 to 16 times their value and fall are off by 9.8e-18 of the largest (RMS, against exact
-// fractions), a chain of FP64 multiply-adds by 5.5e-17, seven slices by 3.0e-16, six by 7.4e-14.
+// 1.9e-10 of the largest coefficient).  Eight slices stay for their precision, 62 bits of each row or
+// column maximum and exact digit sums: sums of 32 products that rise to 5 to 16 times their value and
+// fall are off by 9.8e-18 of the largest (RMS, against exact fractions), a chain of FP64 multiply-adds by
+// 5.5e-17, seven slices by 3.0e-16, six by 7.4e-14.
 namespace {
 void oz_route(const lsd_ctx* c, OzState* o) {
   const double K = (double)c->H / c->M * (c->Th2 & 1 ? 1.15 : 1.0), pad = 48.0 * ceil_div(c->Th2, 48) / c->Th2;
   const int S = o->S;
-  o->synth = S <= 5 || S == 8 || K * pad > (S == 6 ? 122.0 : 175.0);
+  o->synth = S <= 5 || S == 8 || K * pad > (S == 6 ? 130.0 : 175.0);
   o->anal = S <= 5 || S == 8 || K > (S == 6 ? 124.0 : 160.0);
 }
 }  // namespace

@@ -44,8 +44,9 @@ def route(g):
     (208, 32, 1, 7, (True, True)), (204, 128, 1, 7, (True, True)),
     # and 0.4 .. 1.02 times at these
     (128, 16, 1, 6, (False, False)), (192, 192, 1, 6, (False, False)), (192, 32, 6, 6, (False, False)),
-    (256, 256, 1, 7, (False, False)), (192, 96, 1, 7, (False, False)), (256, 32, 8, 7, (False, False)),
-    (192, 64, 1, 7, (False, True)), (153, 48, 1, 7, (True, False)), (64, 16, 4, 7, (False, False)),
+    (256, 256, 1, 6, (False, True)), (256, 256, 1, 7, (False, False)), (192, 96, 1, 7, (False, False)),
+    (256, 32, 8, 7, (False, False)), (192, 64, 1, 7, (False, True)), (153, 48, 1, 7, (True, False)),
+    (64, 16, 4, 7, (False, False)),
     (64, 16, 4, 5, (True, True)), (64, 16, 4, 8, (True, True))])
 def test_faster_side_of_the_dispatch(L, M, Mp, S, int8):
     """also: lsd_create makes the three (synthesis) and two (analysis) digit tables of the directions
